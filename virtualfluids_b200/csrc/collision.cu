@@ -37,6 +37,7 @@ struct CollisionKernelArgs {
     const uint32_t* __restrict__ table;
     K17Rates<R> rates;
     R fx, fy, fz;         // forces * 1/2 * forceFactor
+    bool forced;          // (fx, fy, fz) is not zero
     R gfx, gfy, gfz;      // raw global forces (body-force template)
     R forceFactor;
     R* rho;
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(kCollisionThreads) k17Kernel(const CollisionKe
     for (int d = 0; d < 27; ++d)
         f[d] = Storage<S>::load(a.base[d] + L.k[loc(d)], d);
     R drho, ux, uy, uz;
-    k17Collide<R>(f, a.rates, fx, fy, fz, drho, ux, uy, uz);
+    k17Collide<R>(f, a.rates, fx, fy, fz, drho, ux, uy, uz, BODY_FORCE || a.forced);
     if (WRITE_MACRO) {
         a.vx[k] = ux;
         a.vy[k] = uy;
@@ -402,6 +403,7 @@ static int launchCollision(bool bgk, const vfb_collision_args* a, cudaStream_t s
     k.fx = k.gfx * R(0.5) * k.forceFactor;
     k.fy = k.gfy * R(0.5) * k.forceFactor;
     k.fz = k.gfz * R(0.5) * k.forceFactor;
+    k.forced = !(k.fx == R(0) && k.fy == R(0) && k.fz == R(0));
     k.rho = static_cast<R*>(a->rho);
     k.vx = static_cast<R*>(a->vx);
     k.vy = static_cast<R*>(a->vy);

@@ -3,19 +3,28 @@
 // K17: the compressible cumulant collision of VirtualFluids
 // (src/lbm/collision/K17CompressibleNavierStokes.h:87-591, TurbulenceModel::None),
 // based on Geier et al., J. Comput. Phys. 348 (2017) 862-888 and 889-898.
-// The operator is the reference's, term for term; the arithmetic is arranged
-// for the GPU's issue rate (the step is instruction bound at ~1 kflop/node):
-//   * the chimera transforms are written in multiply-add form with their
-//     conditioning factors multiplied out (algebraically identical);
-//   * density, momentum and the first (z) chimera sweep share the sums over
-//     the nine z lines of the lattice;
+// The operator is the reference's; its arithmetic is arranged for the fewest
+// instructions, because the 16-bit storages and the adjoint are bound by the
+// floating-point pipes (and FP32 by their power):
+//   * orders 4..6 do not depend on their pre-collision values (O4 = O5 = O6 =
+//     1), so only the 17 raw moments up to order 3 are formed, by sums and
+//     differences along z, y and x (no multiplication), and those are shifted
+//     to central moments about the velocity;
+//   * the limiter O + (1 - O) |x| / (|x| + ql) enters as its complement
+//     (1 - O) ql / (|x| + ql), one reciprocal and two multiplications;
+//   * second moments are carried as deviations from rho / 3, in which the
+//     Gaussian closure of orders 4..6 is short and well conditioned
+//     (c200 c020 / rho = rho / 9 + (p + q) / 3 + p q / rho);
+//   * every moment is carried times 1/2 per non-zero exponent, which folds the
+//     halvings of the back transform into the operator's constants;
+//   * the terms of a force are a block of their own, skipped for a launch
+//     without one;
 //   * rates that depend only on omega and the limiters are formed once per
-//     launch on the host (K17Rates) with the reference's expressions;
-//   * cumulants whose post-collision value does not depend on their
-//     pre-collision value (orders 4..6 with O4 = O5 = O6 = 1) are never
-//     formed: the reference computes them and then multiplies them by
-//     (1 - 1) = 0 or cancels them exactly (x + 1 * (-x) = +0);
-//   * in FP32 the seven limiter quotients use the fast division.
+//     launch on the host (K17Rates) with the reference's expressions.
+// Live operations of one node (add, multiply, multiply-add; paired FP32): 450
+// without a force, 470 with one, against 630 of the term-by-term arrangement
+// (forward chimera sweeps on all 27 moments, cumulants by the reference's
+// expressions), counted on a recorded trace.
 // Results agree with the reference to rounding: FP64 fields within 1e-12
 // relative of the oracle after many steps (tests/test_gpu_collision.py).
 //
@@ -41,126 +50,113 @@ __host__ __device__ __forceinline__ R cst(int n, int m)
     return R(S(n) / S(m));
 }
 
-// Per-launch constants of the K17 collision (K17CompressibleNavierStokes.h:245-273,
-// limiter inputs :176-178, force factor RunCollision.cuh:111-113).
+// Per-launch constants of the K17 collision (rates and factors of
+// K17CompressibleNavierStokes.h:245-273 and :452-457, limiter inputs :176-178,
+// combined and scaled as k17Collide uses them):
+//   omega             relaxation rate (the BGK collision's too)
+//   halfMinusOmega    -omega / 2           omegaThreeHalves  3 omega / 2
+//   keepHalf          (1 - omega) / 2      corrHalf          -3/2 (1 - omega / 2)
+//   keep, keepQuarter (1 - omega), (1 - omega) / 4
+//   mixed4            (1 - omega) / 24 + fourthB / 8
+//   limP, limM, limD  (1 - O) ql of the three limiters, over 8, 8 and 2
+//   qlP, qlM, qlD     quartic limiters
+//   fourthA4, minusFourthA4, fourthA24    fourthA / 4, its negative, fourthA / 24
+//   twoFourthB        2 fourthB
+// with fourthA = -(1/omega - 1/2) 2/3 A and fourthB = (1/omega - 1/2) omega B.
+#define VFB_K17_RATES(X)                                                                                               \
+    X(omega) X(halfMinusOmega) X(omegaThreeHalves) X(keepHalf) X(corrHalf) X(keep) X(keepQuarter) X(mixed4) X(limP)    \
+    X(limM) X(limD) X(qlP) X(qlM) X(qlD) X(fourthA4) X(minusFourthA4) X(fourthA24) X(twoFourthB)
+
 template <class R>
 struct K17Rates {
-    R omega;
-    R OxyyPxzz, OxyyMxzz, Oxyz;       // third-order rates
-    R oneMinusOxyyPxzz, oneMinusOxyyMxzz, oneMinusOxyz;
-    R factorA, factorB;               // fourth-order modified equilibrium
-    R minusTau;                       // -O4 * (1/omega - 1/2)
-    R halfMinusOmega;                 // 1/2 * (-omega)
-    R omegaThreeHalves;               // omega * 3/2
-    R minusThreeOmega;                // -3 * omega
-    R secondOrderCorrection;          // 3 * (1 + 1/2 * (-omega))
-    R qlP, qlM, qlD;                  // quartic limiters
-    // per-launch factors of the fourth-order terms (:452-457):
-    // minusTau * 2/3 * factorA, minusTau * (-3 omega) * 1/3 * factorB
-    R fourthA, fourthB;
+#define VFB_FIELD(name) R name;
+    VFB_K17_RATES(VFB_FIELD)
+#undef VFB_FIELD
 };
+
+// A limiter above 2^60 (infinity too) leaves a moment's rate at O to rounding,
+// one below 2^-100 relaxes it fully; inside these bounds the products with ql
+// and the reciprocal stay finite in FP32.
+template <class R>
+inline R boundedLimiter(R ql)
+{
+    const R hi = R(1152921504606846976.0), lo = R(7.888609052210118e-31);
+    return ql > hi ? hi : ql >= R(0) && ql < lo ? lo : ql;
+}
 
 template <class R>
 inline K17Rates<R> makeK17Rates(R omega, R qlP, R qlM, R qlD)
 {
     K17Rates<R> r;
     r.omega = omega;
-    r.OxyyPxzz = R(8) * (-R(2) + omega) * (R(1) + R(2) * omega) / (-R(8) - R(14) * omega + R(7) * omega * omega);
-    r.OxyyMxzz = R(8) * (-R(2) + omega) * (-R(7) + R(4) * omega) / (R(56) - R(50) * omega + R(9) * omega * omega);
-    r.Oxyz = R(24) * (-R(2) + omega) * (-R(2) - R(7) * omega + R(3) * omega * omega) /
-             (R(48) + R(152) * omega - R(130) * omega * omega + R(29) * omega * omega * omega);
-    r.oneMinusOxyyPxzz = R(1) - r.OxyyPxzz;
-    r.oneMinusOxyyMxzz = R(1) - r.OxyyMxzz;
-    r.oneMinusOxyz = R(1) - r.Oxyz;
-    r.factorA = (R(4) + R(2) * omega - R(3) * omega * omega) / (R(2) - R(7) * omega + R(5) * omega * omega);
-    r.factorB = (R(4) + R(28) * omega - R(14) * omega * omega) / (R(6) - R(21) * omega + R(15) * omega * omega);
-    r.minusTau = -R(1) * (R(1) / omega - cst<R>(1, 2));
+    const R OxyyPxzz = R(8) * (-R(2) + omega) * (R(1) + R(2) * omega) / (-R(8) - R(14) * omega + R(7) * omega * omega);
+    const R OxyyMxzz =
+        R(8) * (-R(2) + omega) * (-R(7) + R(4) * omega) / (R(56) - R(50) * omega + R(9) * omega * omega);
+    const R Oxyz = R(24) * (-R(2) + omega) * (-R(2) - R(7) * omega + R(3) * omega * omega) /
+                   (R(48) + R(152) * omega - R(130) * omega * omega + R(29) * omega * omega * omega);
+    const R factorA = (R(4) + R(2) * omega - R(3) * omega * omega) / (R(2) - R(7) * omega + R(5) * omega * omega);
+    const R factorB = (R(4) + R(28) * omega - R(14) * omega * omega) / (R(6) - R(21) * omega + R(15) * omega * omega);
+    const R minusTau = -R(1) * (R(1) / omega - cst<R>(1, 2));
+    const R fourthA = minusTau * cst<R>(2, 3) * factorA;
+    const R fourthB = minusTau * (-R(3) * omega) * cst<R>(1, 3) * factorB;
     r.halfMinusOmega = cst<R>(1, 2) * (-omega);
     r.omegaThreeHalves = omega * (cst<R>(3, 2));
-    r.minusThreeOmega = -R(3) * omega;
-    r.secondOrderCorrection = R(3) * (R(1) + cst<R>(1, 2) * (-omega));
-    r.qlP = qlP;
-    r.qlM = qlM;
-    r.qlD = qlD;
-    r.fourthA = r.minusTau * cst<R>(2, 3) * r.factorA;
-    r.fourthB = r.minusTau * r.minusThreeOmega * cst<R>(1, 3) * r.factorB;
+    r.keep = R(1) - omega;
+    r.keepHalf = r.keep * R(0.5);
+    r.keepQuarter = r.keep * R(0.25);
+    r.corrHalf = -cst<R>(3, 2) * (R(1) + cst<R>(1, 2) * (-omega));
+    r.mixed4 = r.keep * cst<R>(1, 24) + fourthB * R(0.125);
+    r.qlP = boundedLimiter(qlP);
+    r.qlM = boundedLimiter(qlM);
+    r.qlD = boundedLimiter(qlD);
+    r.limP = (R(1) - OxyyPxzz) * r.qlP * R(0.125);
+    r.limM = (R(1) - OxyyMxzz) * r.qlM * R(0.125);
+    r.limD = (R(1) - Oxyz) * r.qlD * R(0.5);
+    r.fourthA4 = fourthA * R(0.25);
+    r.minusFourthA4 = -r.fourthA4;
+    r.fourthA24 = fourthA * cst<R>(1, 24);
+    r.twoFourthB = R(2) * fourthB;
     return r;
 }
 
-// ---------------------------------------------------------------- chimera --
-// Central-moment transforms of ChimeraTransformation.h:58-121 (Geier et al.
-// 2015, appendix J), written in multiply-add form.  With the conditioning pair
-// (Kinverse, K) of a line and Kq = Kinverse * K:
-//   forward   a' = a + b + c
-//             b' = Kq (m1 - vv m0) - K vv,      m1 = c - a, m2 = a + c, m0 = a'
-//             c' = Kq (m2 - 2 vv m1 + v2 m0) + K v2
-//   backward  a' = c/2 + b (vv - 1/2) + (a + K) (v2 - vv)/2
-//             b' = (a - c) - 2 vv b - v2 (a + K)
-//             c' = c/2 + b (vv + 1/2) + (a + K) (v2 + vv)/2
-// which are the reference's expressions with the factors Kinverse and K
-// multiplied out (every line has Kq = 1 except the last forward x line, whose
-// pair (3, 1/9) gives Kq = 1/3; K = 0 gives the plain transforms).
+// -------------------------------------------------------------- transforms --
+// Raw moments of order 0, 1, 2 of one lattice line (a, b, c) = (-1, 0, +1), in
+// place: sums and differences only.
+template <class R>
+__host__ __device__ __forceinline__ void lineMoments(R& a, R& b, R& c)
+{
+    const R m2 = a + c;
+    const R m1 = c - a;
+    a = m2 + b;
+    b = m1;
+    c = m2;
+}
+
+// The back transform of one line: central moments (a, b, c) of order 0, 1, 2
+// about the velocity v to the line's populations, the inverse of
+// ChimeraTransformation.h:58-121 (Geier et al. 2015, appendix J) with the
+// equilibrium part K of the zeroth moment.  b and c come as halves: with
+//   r1 = (b + v (a + K)) / 2,   r2 = (c + v b + v (b + v (a + K))) / 2
+// half the raw moments, the populations are r2 - r1, a - 2 r2 and r2 + r1.
 template <class R>
 struct Sweep {
-    R vv, v2, nvv, n2vv, nv2, hm, hp, vvm, vvp;
-    __host__ __device__ __forceinline__ Sweep(R v)
+    R v, half;
+    __host__ __device__ __forceinline__ Sweep(R velocity)
     {
-        vv = v;
-        v2 = v * v;
-        nvv = -v;
-        n2vv = R(-2) * v;
-        nv2 = -v2;
-        hm = R(0.5) * (v2 - v);
-        hp = R(0.5) * (v2 + v);
-        vvm = v - R(0.5);
-        vvp = v + R(0.5);
+        v = velocity;
+        half = R(0.5) * velocity;
     }
 };
-
-template <class R>
-__host__ __device__ __forceinline__ void fwd(R& a, R& b, R& c, const Sweep<R>& w, typename ScalarOf<R>::type K)
-{
-    const R m2 = a + c;
-    const R m1 = c - a;
-    const R m0 = m2 + b;
-    const R m0K = K != 0 ? m0 + R(K) : m0;
-    a = m0;
-    b = fma(w.nvv, m0K, m1);
-    c = fma(w.v2, m0K, fma(w.n2vv, m1, m2));
-}
-
-// the forward x line with (Kinverse, K) = (3, 1/9) of K17CompressibleNavierStokes.h:222
-template <class R>
-__host__ __device__ __forceinline__ void fwdThird(R& a, R& b, R& c, const Sweep<R>& w)
-{
-    const R m2 = a + c;
-    const R m1 = c - a;
-    const R m0 = m2 + b;
-    a = m0;
-    b = fma(cst<R>(1, 3), fma(w.nvv, m0, m1), w.nvv * (cst<R>(1, 9)));
-    c = fma(cst<R>(1, 3), fma(w.v2, m0, fma(w.n2vv, m1, m2)), w.v2 * (cst<R>(1, 9)));
-}
 
 template <class R>
 __host__ __device__ __forceinline__ void bwd(R& a, R& b, R& c, const Sweep<R>& w, typename ScalarOf<R>::type K)
 {
     const R aK = K != 0 ? a + R(K) : a;
-    const R hc = R(0.5) * c;
-    const R na = fma(aK, w.hm, fma(b, w.vvm, hc));
-    if constexpr (sizeof(typename ScalarOf<R>::type) == 8) {
-        // FP64: three independent chains (measured faster in double precision)
-        const R nb = fma(w.nv2, aK, fma(w.n2vv, b, a - c));
-        c = fma(aK, w.hp, fma(b, w.vvp, hc));
-        a = na;
-        b = nb;
-    } else {
-        // FP32 (scalar or paired): two operations fewer; hp - hm = v and
-        // vvp - vvm = 1, and the three populations sum to a
-        const R nc = na + fma(aK, w.vv, b);
-        b = (a - na) - nc;
-        a = na;
-        c = nc;
-    }
+    const R r1 = fma(w.half, aK, b);
+    const R r2 = fma(w.v, b + r1, c);
+    b = fma(R(-2), r2, a);
+    a = r2 - r1;
+    c = r2 + r1;
 }
 
 // --------------------------------------------------------- macroscopic sums --
@@ -197,174 +193,119 @@ __host__ __device__ __forceinline__ R pyramidJz(const R* f)
 }
 
 // ------------------------------------------------------------------- K17 --
-// sixth-order correction term of K17CompressibleNavierStokes.h:320-330 / :489-500,
-// regrouped as (A + B / rho) / rho: A collects the terms over rho, B those
-// over rho^2 (the same terms, fused multiply-adds)
+// 1 / x of the density.
 template <class R>
-__host__ __device__ __forceinline__ R c222Term(R m111, R m200, R m020, R m002, R m022, R m202, R m220, R m011, R m101, R m110,
-                                      R m211, R m121, R m112, R m120, R m102, R m210, R m012, R m201, R m021,
-                                      R oneOverRho, R drho)
+__host__ __device__ __forceinline__ R reciprocal(R x)
 {
-    const R s2 = m200 + m020 + m002;
-    const R a1 = fma(m002, m220, fma(m020, m202, m200 * m022));
-    const R a2 = fma(m110, m112, fma(m101, m121, m011 * m211));
-    const R a3 = fma(m201, m021, fma(m210, m012, m120 * m102));
-    R A = fma(R(-4), m111 * m111, -a1);
-    A = fma(R(-4), a2, A);
-    A = fma(R(-2), a3, A);
-    A = fma(-cst<R>(1, 3), m022 + m202 + m220, A);
-    A = fma(-cst<R>(1, 9), s2, A);
-    const R q101 = m101 * m101, q011 = m011 * m011, q110 = m110 * m110;
-    const R m200m020 = m200 * m020;
-    const R b1 = fma(q110, m002, fma(q011, m200, q101 * m020));
-    const R pairs = fma(m002, m020, fma(m002, m200, m200m020));
-    const R inner = fma(cst<R>(1, 3), s2, fma(R(2), q101 + q011 + q110, pairs));
-    R B = fma(R(2), m200m020 * m002, R(4) * b1);
-    B = fma(R(16), (m110 * m101) * m011, B);
-    B = fma(cst<R>(2, 3), inner, B);
-    B = fma(cst<R>(1, 27), fma(drho, drho, -drho), B);
-    return fma(B, oneOverRho, A) * oneOverRho;
+    return R(1) / x;
 }
-
+// 1 / x of a limiter's denominator: in FP32 the hardware's approximate
+// reciprocal (relative error about 1e-7 of a moment that is a small part of
+// the populations)
 template <class R>
-__host__ __device__ __forceinline__ R limiterQuotient(R x, R y)
+__host__ __device__ __forceinline__ R limiterReciprocal(R x)
 {
-    return x / y;
+    return R(1) / x;
 }
 #ifdef __CUDA_ARCH__
-template <>
-__device__ __forceinline__ float limiterQuotient<float>(float x, float y)
+__device__ __forceinline__ float approximateReciprocal(float x)
 {
-    return __fdividef(x, y);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// one Newton-Raphson step r (2 - x r) on the approximate reciprocal
+template <>
+__device__ __forceinline__ float reciprocal<float>(float x)
+{
+    const float r = approximateReciprocal(x);
+    return fmaf(fmaf(-x, r, 1.0f), r, r);
+}
+template <>
+__device__ __forceinline__ float limiterReciprocal<float>(float x)
+{
+    return approximateReciprocal(x);
 }
 #endif
 
-// Central moments (in the slots of k17Collide's naming: m_abc in the slot of
-// direction (a-1, b-1, c-1)) to populations: the backward chimera transform
-// in x, then y, then z (K17CompressibleNavierStokes.h:525-557; the same
-// sequence closes the interface interpolation, InterpolationCF.h:250-285).
+// a third-order combination x relaxed by its limited rate: x (1 - O) ql / (|x| + ql)
 template <class R>
-__host__ __device__ __forceinline__ void centralMomentsToPopulations(R* f, R vvx, R vvy, R vvz)
+__host__ __device__ __forceinline__ R limitedMoment(R x, R lim, R ql)
 {
+    return (x * lim) * limiterReciprocal(fabs(x) + ql);
+}
+
+// Central moments, scaled by 1/2 per non-zero exponent (in the slots of
+// k17Collide's naming: m_abc in the slot of direction (a-1, b-1, c-1)), to
+// populations: the back transform in x, then y, then z
+// (K17CompressibleNavierStokes.h:525-557).  The equilibrium parts K carry the
+// scale of their line.
+template <class R>
+__host__ __device__ __forceinline__ void scaledMomentsToPopulations(R* f, R vvx, R vvy, R vvz)
+{
+    using S = typename ScalarOf<R>::type;
     {
         const Sweep<R> w(vvx);
-        bwd(f[dMMM], f[d0MM], f[dPMM], w, typename ScalarOf<R>::type(1));
-        bwd(f[dM0M], f[d00M], f[dP0M], w, typename ScalarOf<R>::type(0));
-        bwd(f[dMPM], f[d0PM], f[dPPM], w, cst<typename ScalarOf<R>::type>(1, 3));
-        bwd(f[dMM0], f[d0M0], f[dPM0], w, typename ScalarOf<R>::type(0));
-        bwd(f[dM00], f[d000], f[dP00], w, typename ScalarOf<R>::type(0));
-        bwd(f[dMP0], f[d0P0], f[dPP0], w, typename ScalarOf<R>::type(0));
-        bwd(f[dMMP], f[d0MP], f[dPMP], w, cst<typename ScalarOf<R>::type>(1, 3));
-        bwd(f[dM0P], f[d00P], f[dP0P], w, typename ScalarOf<R>::type(0));
-        bwd(f[dMPP], f[d0PP], f[dPPP], w, cst<typename ScalarOf<R>::type>(1, 9));
+        bwd(f[dMMM], f[d0MM], f[dPMM], w, S(1));
+        bwd(f[dM0M], f[d00M], f[dP0M], w, S(0));
+        bwd(f[dMPM], f[d0PM], f[dPPM], w, cst<S>(1, 6));
+        bwd(f[dMM0], f[d0M0], f[dPM0], w, S(0));
+        bwd(f[dM00], f[d000], f[dP00], w, S(0));
+        bwd(f[dMP0], f[d0P0], f[dPP0], w, S(0));
+        bwd(f[dMMP], f[d0MP], f[dPMP], w, cst<S>(1, 6));
+        bwd(f[dM0P], f[d00P], f[dP0P], w, S(0));
+        bwd(f[dMPP], f[d0PP], f[dPPP], w, cst<S>(1, 36));
     }
     {
         const Sweep<R> w(vvy);
-        bwd(f[dMMM], f[dM0M], f[dMPM], w, cst<typename ScalarOf<R>::type>(1, 6));
-        bwd(f[dMM0], f[dM00], f[dMP0], w, typename ScalarOf<R>::type(0));
-        bwd(f[dMMP], f[dM0P], f[dMPP], w, cst<typename ScalarOf<R>::type>(1, 18));
-        bwd(f[d0MM], f[d00M], f[d0PM], w, cst<typename ScalarOf<R>::type>(2, 3));
-        bwd(f[d0M0], f[d000], f[d0P0], w, typename ScalarOf<R>::type(0));
-        bwd(f[d0MP], f[d00P], f[d0PP], w, cst<typename ScalarOf<R>::type>(2, 9));
-        bwd(f[dPMM], f[dP0M], f[dPPM], w, cst<typename ScalarOf<R>::type>(1, 6));
-        bwd(f[dPM0], f[dP00], f[dPP0], w, typename ScalarOf<R>::type(0));
-        bwd(f[dPMP], f[dP0P], f[dPPP], w, cst<typename ScalarOf<R>::type>(1, 18));
+        bwd(f[dMMM], f[dM0M], f[dMPM], w, cst<S>(1, 6));
+        bwd(f[dMM0], f[dM00], f[dMP0], w, S(0));
+        bwd(f[dMMP], f[dM0P], f[dMPP], w, cst<S>(1, 36));
+        bwd(f[d0MM], f[d00M], f[d0PM], w, cst<S>(2, 3));
+        bwd(f[d0M0], f[d000], f[d0P0], w, S(0));
+        bwd(f[d0MP], f[d00P], f[d0PP], w, cst<S>(1, 9));
+        bwd(f[dPMM], f[dP0M], f[dPPM], w, cst<S>(1, 6));
+        bwd(f[dPM0], f[dP00], f[dPP0], w, S(0));
+        bwd(f[dPMP], f[dP0P], f[dPPP], w, cst<S>(1, 36));
     }
     {
         const Sweep<R> w(vvz);
-        bwd(f[dMMM], f[dMM0], f[dMMP], w, cst<typename ScalarOf<R>::type>(1, 36));
-        bwd(f[dM0M], f[dM00], f[dM0P], w, cst<typename ScalarOf<R>::type>(1, 9));
-        bwd(f[dMPM], f[dMP0], f[dMPP], w, cst<typename ScalarOf<R>::type>(1, 36));
-        bwd(f[d0MM], f[d0M0], f[d0MP], w, cst<typename ScalarOf<R>::type>(1, 9));
-        bwd(f[d00M], f[d000], f[d00P], w, cst<typename ScalarOf<R>::type>(4, 9));
-        bwd(f[d0PM], f[d0P0], f[d0PP], w, cst<typename ScalarOf<R>::type>(1, 9));
-        bwd(f[dPMM], f[dPM0], f[dPMP], w, cst<typename ScalarOf<R>::type>(1, 36));
-        bwd(f[dP0M], f[dP00], f[dP0P], w, cst<typename ScalarOf<R>::type>(1, 9));
-        bwd(f[dPPM], f[dPP0], f[dPPP], w, cst<typename ScalarOf<R>::type>(1, 36));
+        bwd(f[dMMM], f[dMM0], f[dMMP], w, cst<S>(1, 36));
+        bwd(f[dM0M], f[dM00], f[dM0P], w, cst<S>(1, 9));
+        bwd(f[dMPM], f[dMP0], f[dMPP], w, cst<S>(1, 36));
+        bwd(f[d0MM], f[d0M0], f[d0MP], w, cst<S>(1, 9));
+        bwd(f[d00M], f[d000], f[d00P], w, cst<S>(4, 9));
+        bwd(f[d0PM], f[d0P0], f[d0PP], w, cst<S>(1, 9));
+        bwd(f[dPMM], f[dPM0], f[dPMP], w, cst<S>(1, 36));
+        bwd(f[dP0M], f[dP00], f[dP0P], w, cst<S>(1, 9));
+        bwd(f[dPPM], f[dPP0], f[dPPP], w, cst<S>(1, 36));
     }
+}
+
+// the same from unscaled central moments (the interface interpolation,
+// InterpolationCF.h:250-285): exact scalings first
+template <class R>
+__host__ __device__ __forceinline__ void centralMomentsToPopulations(R* f, R vvx, R vvy, R vvz)
+{
+#pragma unroll
+    for (int d = 0; d < 27; ++d) {
+        // the moment in the slot of direction d has a non-zero exponent on the axes where c_d >= 0
+        const int nz = (cx(d) >= 0) + (cy(d) >= 0) + (cz(d) >= 0);
+        if (nz)
+            f[d] = f[d] * R(nz == 1 ? 0.5 : nz == 2 ? 0.25 : 0.125);
+    }
+    scaledMomentsToPopulations(f, vvx, vvy, vvz);
 }
 
 // One K17 collision on f[27] (pre-collision in, post-collision out).
 // (fx, fy, fz) is half the acceleration already scaled by the level factor
-// (RunCollision.cuh:111-113).  Returns drho and the force-shifted velocity.
+// (RunCollision.cuh:111-113); forced = false promises that it is zero.
+// Returns drho and the force-shifted velocity.
 template <class R>
 __host__ __device__ __forceinline__ void k17Collide(R* f, const K17Rates<R>& r, R fx, R fy, R fz, R& drho_out,
-                                                    R& vx_out, R& vy_out, R& vz_out)
+                                                    R& vx_out, R& vy_out, R& vz_out, bool forced = true)
 {
-    // sums over the nine z lines (x, y fixed): s = a + b + c, m2 = a + c, d = c - a
-#define VFB_ZLINE(XY, A, B, C)                                                                                         \
-    const R m2_##XY = f[A] + f[C];                                                                                     \
-    const R d_##XY = f[C] - f[A];                                                                                      \
-    const R s_##XY = m2_##XY + f[B];
-    VFB_ZLINE(MM, dMMM, dMM0, dMMP)
-    VFB_ZLINE(M0, dM0M, dM00, dM0P)
-    VFB_ZLINE(MP, dMPM, dMP0, dMPP)
-    VFB_ZLINE(0M, d0MM, d0M0, d0MP)
-    VFB_ZLINE(00, d00M, d000, d00P)
-    VFB_ZLINE(0P, d0PM, d0P0, d0PP)
-    VFB_ZLINE(PM, dPMM, dPM0, dPMP)
-    VFB_ZLINE(P0, dP0M, dP00, dP0P)
-    VFB_ZLINE(PP, dPPM, dPP0, dPPP)
-#undef VFB_ZLINE
-    const R drho = (((s_MM + s_PP) + (s_MP + s_PM)) + ((s_M0 + s_P0) + (s_0M + s_0P))) + s_00;
-    const R jx = ((s_PM + s_PP) - (s_MM + s_MP)) + (s_P0 - s_M0);
-    const R jy = ((s_MP + s_PP) - (s_MM + s_PM)) + (s_0P - s_0M);
-    const R jz = (((d_MM + d_PP) + (d_MP + d_PM)) + ((d_M0 + d_P0) + (d_0M + d_0P))) + d_00;
-    const R oneOverRho = R(1) / (drho + R(1));
-    const R vvx = fma(jx, oneOverRho, fx);
-    const R vvy = fma(jy, oneOverRho, fy);
-    const R vvz = fma(jz, oneOverRho, fz);
-    const R vx2 = vvx * vvx, vy2 = vvy * vvy, vz2 = vvz * vvz;
-
-    // forward chimera in z (:190-199) from the line sums
-    {
-        const Sweep<R> w(vvz);
-#define VFB_ZFWD(XY, A, B, C, K)                                                                                       \
-    {                                                                                                                  \
-        const R m0K = s_##XY + (K);                                                                                    \
-        f[A] = s_##XY;                                                                                                 \
-        f[B] = fma(w.nvv, m0K, d_##XY);                                                                                \
-        f[C] = fma(w.v2, m0K, fma(w.n2vv, d_##XY, m2_##XY));                                                           \
-    }
-        VFB_ZFWD(MM, dMMM, dMM0, dMMP, cst<R>(1, 36))
-        VFB_ZFWD(M0, dM0M, dM00, dM0P, cst<R>(1, 9))
-        VFB_ZFWD(MP, dMPM, dMP0, dMPP, cst<R>(1, 36))
-        VFB_ZFWD(0M, d0MM, d0M0, d0MP, cst<R>(1, 9))
-        VFB_ZFWD(00, d00M, d000, d00P, cst<R>(4, 9))
-        VFB_ZFWD(0P, d0PM, d0P0, d0PP, cst<R>(1, 9))
-        VFB_ZFWD(PM, dPMM, dPM0, dPMP, cst<R>(1, 36))
-        VFB_ZFWD(P0, dP0M, dP00, dP0P, cst<R>(1, 9))
-        VFB_ZFWD(PP, dPPM, dPP0, dPPP, cst<R>(1, 36))
-#undef VFB_ZFWD
-    }
-    // y (:202-210)
-    {
-        const Sweep<R> w(vvy);
-        fwd(f[dMMM], f[dM0M], f[dMPM], w, cst<typename ScalarOf<R>::type>(1, 6));
-        fwd(f[dMM0], f[dM00], f[dMP0], w, typename ScalarOf<R>::type(0));
-        fwd(f[dMMP], f[dM0P], f[dMPP], w, cst<typename ScalarOf<R>::type>(1, 18));
-        fwd(f[d0MM], f[d00M], f[d0PM], w, cst<typename ScalarOf<R>::type>(2, 3));
-        fwd(f[d0M0], f[d000], f[d0P0], w, typename ScalarOf<R>::type(0));
-        fwd(f[d0MP], f[d00P], f[d0PP], w, cst<typename ScalarOf<R>::type>(2, 9));
-        fwd(f[dPMM], f[dP0M], f[dPPM], w, cst<typename ScalarOf<R>::type>(1, 6));
-        fwd(f[dPM0], f[dP00], f[dPP0], w, typename ScalarOf<R>::type(0));
-        fwd(f[dPMP], f[dP0P], f[dPPP], w, cst<typename ScalarOf<R>::type>(1, 18));
-    }
-    // x (:213-222)
-    {
-        const Sweep<R> w(vvx);
-        fwd(f[dMMM], f[d0MM], f[dPMM], w, typename ScalarOf<R>::type(1));
-        fwd(f[dM0M], f[d00M], f[dP0M], w, typename ScalarOf<R>::type(0));
-        fwd(f[dMPM], f[d0PM], f[dPPM], w, cst<typename ScalarOf<R>::type>(1, 3));
-        fwd(f[dMM0], f[d0M0], f[dPM0], w, typename ScalarOf<R>::type(0));
-        fwd(f[dM00], f[d000], f[dP00], w, typename ScalarOf<R>::type(0));
-        fwd(f[dMP0], f[d0P0], f[dPP0], w, typename ScalarOf<R>::type(0));
-        fwd(f[dMMP], f[d0MP], f[dPMP], w, cst<typename ScalarOf<R>::type>(1, 3));
-        fwd(f[dM0P], f[d00P], f[dP0P], w, typename ScalarOf<R>::type(0));
-        fwdThird(f[dMPP], f[d0PP], f[dPPP], w);
-    }
-
-    // moment names: m_abc is stored in the slot of direction (a-1, b-1, c-1)
+    // moment names: m_abc (x^a y^b z^c) in the slot of direction (a-1, b-1, c-1)
     R& m000 = f[dMMM];
     R& m100 = f[d0MM];
     R& m200 = f[dPMM];
@@ -393,97 +334,169 @@ __host__ __device__ __forceinline__ void k17Collide(R* f, const K17Rates<R>& r, 
     R& m122 = f[d0PP];
     R& m222 = f[dPPP];
 
-    // second and third order combinations (:329-346)
-    R mxxPyyPzz = m200 + m020 + m002;
-    R mxxMyy = m200 - m020;
-    R mxxMzz = m200 - m002;
-    R mxxyPyzz = m210 + m012;
-    R mxxyMyzz = m210 - m012;
-    R mxxzPyyz = m201 + m021;
-    R mxxzMyyz = m201 - m021;
-    R mxyyPxzz = m120 + m102;
-    R mxyyMxzz = m120 - m102;
+    // raw moments of the deviations, axis by axis (those above order 3 are
+    // never used and cost nothing)
+    lineMoments(f[dMMM], f[dMM0], f[dMMP]);
+    lineMoments(f[dM0M], f[dM00], f[dM0P]);
+    lineMoments(f[dMPM], f[dMP0], f[dMPP]);
+    lineMoments(f[d0MM], f[d0M0], f[d0MP]);
+    lineMoments(f[d00M], f[d000], f[d00P]);
+    lineMoments(f[d0PM], f[d0P0], f[d0PP]);
+    lineMoments(f[dPMM], f[dPM0], f[dPMP]);
+    lineMoments(f[dP0M], f[dP00], f[dP0P]);
+    lineMoments(f[dPPM], f[dPP0], f[dPPP]);
 
-    // velocity gradients (:357-362), OxxPyyPzz = 1; the mixed ones (from the
-    // second-order moments before relaxation) enter only the fourth-order
-    // terms, through fourthB
-    const R cm112 = r.fourthB * m110;
-    const R cm121 = r.fourthB * m101;
-    const R cm211 = r.fourthB * m011;
-    const R dxux = r.halfMinusOmega * (mxxMyy + mxxMzz) + R(0.5) * (m000 - mxxPyyPzz);
-    const R dyuy = dxux + r.omegaThreeHalves * mxxMyy;
-    const R dzuz = dxux + r.omegaThreeHalves * mxxMzz;
+    lineMoments(f[dMMM], f[dM0M], f[dMPM]);
+    lineMoments(f[dMM0], f[dM00], f[dMP0]);
+    lineMoments(f[dMMP], f[dM0P], f[dMPP]);
+    lineMoments(f[d0MM], f[d00M], f[d0PM]);
+    lineMoments(f[d0M0], f[d000], f[d0P0]);
+    lineMoments(f[d0MP], f[d00P], f[d0PP]);
+    lineMoments(f[dPMM], f[dP0M], f[dPPM]);
+    lineMoments(f[dPM0], f[dP00], f[dPP0]);
+    lineMoments(f[dPMP], f[dP0P], f[dPPP]);
 
-    // second order relaxation with correction (:387-389)
-    mxxPyyPzz += (m000 - mxxPyyPzz) - R(1.5) * (vx2 * dxux + vy2 * dyuy + vz2 * dzuz);
-    mxxMyy += r.omega * (-mxxMyy) - r.secondOrderCorrection * (vx2 * dxux - vy2 * dyuy);
-    mxxMzz += r.omega * (-mxxMzz) - r.secondOrderCorrection * (vx2 * dxux - vz2 * dzuz);
-    m011 += r.omega * (-m011);
-    m101 += r.omega * (-m101);
-    m110 += r.omega * (-m110);
+    lineMoments(f[dMMM], f[d0MM], f[dPMM]);
+    lineMoments(f[dM0M], f[d00M], f[dP0M]);
+    lineMoments(f[dMPM], f[d0PM], f[dPPM]);
+    lineMoments(f[dMM0], f[d0M0], f[dPM0]);
+    lineMoments(f[dM00], f[d000], f[dP00]);
+    lineMoments(f[dMP0], f[d0P0], f[dPP0]);
+    lineMoments(f[dMMP], f[d0MP], f[dPMP]);
+    lineMoments(f[dM0P], f[d00P], f[dP0P]);
 
-    // third order with quartic limiter (:404-417)
-    R w;
-    w = fma(r.oneMinusOxyz, limiterQuotient(fabs(m111), fabs(m111) + r.qlD), r.Oxyz);
-    m111 += w * (-m111);
-    w = fma(r.oneMinusOxyyPxzz, limiterQuotient(fabs(mxxyPyzz), fabs(mxxyPyzz) + r.qlP), r.OxyyPxzz);
-    mxxyPyzz += w * (-mxxyPyzz);
-    w = fma(r.oneMinusOxyyMxzz, limiterQuotient(fabs(mxxyMyzz), fabs(mxxyMyzz) + r.qlM), r.OxyyMxzz);
-    mxxyMyzz += w * (-mxxyMyzz);
-    w = fma(r.oneMinusOxyyPxzz, limiterQuotient(fabs(mxxzPyyz), fabs(mxxzPyyz) + r.qlP), r.OxyyPxzz);
-    mxxzPyyz += w * (-mxxzPyyz);
-    w = fma(r.oneMinusOxyyMxzz, limiterQuotient(fabs(mxxzMyyz), fabs(mxxzMyyz) + r.qlM), r.OxyyMxzz);
-    mxxzMyyz += w * (-mxxzMyyz);
-    w = fma(r.oneMinusOxyyPxzz, limiterQuotient(fabs(mxyyPxzz), fabs(mxyyPxzz) + r.qlP), r.OxyyPxzz);
-    mxyyPxzz += w * (-mxyyPxzz);
-    w = fma(r.oneMinusOxyyMxzz, limiterQuotient(fabs(mxyyMxzz), fabs(mxyyMxzz) + r.qlM), r.OxyyMxzz);
-    mxyyMxzz += w * (-mxyyMxzz);
+    const R drho = m000;
+    const R rho = drho + R(1);
+    const R oneOverRho = reciprocal(rho);
+    const R vvx = fma(m100, oneOverRho, fx);
+    const R vvy = fma(m010, oneOverRho, fy);
+    const R vvz = fma(m001, oneOverRho, fz);
+    const R nx = -vvx, ny = -vvy, nz = -vvz;
+    const R vx2 = vvx * vvx, vy2 = vvy * vvy, vz2 = vvz * vvz;
 
-    // back to single moments (:431-441)
-    // (1/3)(-2 a + b + c) = (1/3)(a + b + c) - a, likewise for m002
-    m200 = cst<R>(1, 3) * (mxxMyy + mxxMzz + mxxPyyPzz);
-    m020 = m200 - mxxMyy;
-    m002 = m200 - mxxMzz;
-    m210 = (mxxyMyzz + mxxyPyzz) * R(0.5);
-    m012 = (-mxxyMyzz + mxxyPyzz) * R(0.5);
-    m201 = (mxxzMyyz + mxxzPyyz) * R(0.5);
-    m021 = (-mxxzMyyz + mxxzPyyz) * R(0.5);
-    m120 = (mxyyMxzz + mxyyPxzz) * R(0.5);
-    m102 = (-mxyyMxzz + mxyyPxzz) * R(0.5);
+    // central moments about v.  Second order (with j the momentum):
+    //   c200 = m200 - vx jx,  c110 = m110 - vx jy
+    // third order, with the raw second moments M = m + 1/3 and m011:
+    //   c210 = m210 - vy M200 - 2 vx c110,  c111 = m111 - vx m011 - vy c101 - vz c110
+    const R raw200 = m200 + cst<R>(1, 3), raw020 = m020 + cst<R>(1, 3), raw002 = m002 + cst<R>(1, 3);
+    const R raw011 = m011;
+    m200 = fma(nx, m100, m200);
+    m020 = fma(ny, m010, m020);
+    m002 = fma(nz, m001, m002);
+    m110 = fma(nx, m010, m110);
+    m101 = fma(nx, m001, m101);
+    m011 = fma(ny, m001, m011);
+    // with a force the first central moments are -rho (fx, fy, fz): their
+    // contributions to the shifts, and their changed signs after the collision (:512-514)
+    m100 = R(0);
+    m010 = R(0);
+    m001 = R(0);
+    if (forced) {
+        const R gx = rho * fx, gy = rho * fy, gz = rho * fz;
+        m200 = fma(vvx, gx, m200);
+        m020 = fma(vvy, gy, m020);
+        m002 = fma(vvz, gz, m002);
+        m110 = fma(vvy, gx, m110);
+        m101 = fma(vvz, gx, m101);
+        m011 = fma(vvz, gy, m011);
+        m210 = fma(vx2, gy, m210);
+        m201 = fma(vx2, gz, m201);
+        m120 = fma(vy2, gx, m120);
+        m021 = fma(vy2, gz, m021);
+        m102 = fma(vz2, gx, m102);
+        m012 = fma(vz2, gy, m012);
+        m111 = fma(vvy * vvz, gx, m111);
+        m100 = R(0.5) * gx;
+        m010 = R(0.5) * gy;
+        m001 = R(0.5) * gz;
+    }
+    const R n2x = nx + nx, n2y = ny + ny, n2z = nz + nz;
+    m210 = fma(n2x, m110, fma(ny, raw200, m210));
+    m201 = fma(n2x, m101, fma(nz, raw200, m201));
+    m120 = fma(n2y, m110, fma(nx, raw020, m120));
+    m021 = fma(n2y, m011, fma(nz, raw020, m021));
+    m102 = fma(n2z, m101, fma(nx, raw002, m102));
+    m012 = fma(n2z, m011, fma(ny, raw002, m012));
+    m111 = fma(nz, m110, fma(ny, m101, fma(nx, raw011, m111)));
 
-    // fourth order to the modified equilibrium (:452-457); orders 5 and 6
-    // relax to zero (:463-471)
-    const R cm022 = r.fourthA * (dyuy + dzuz);
-    const R cm202 = r.fourthA * (dxux + dzuz);
-    const R cm220 = r.fourthA * (dyuy + dxux);
+    // velocity gradients (:357-362), OxxPyyPzz = 1
+    const R mxxMyy = m200 - m020;
+    const R mxxMzz = m200 - m002;
+    const R nonEq = drho - (m200 + m020 + m002);
+    const R dxux = fma(r.halfMinusOmega, mxxMyy + mxxMzz, R(0.5) * nonEq);
+    const R dyuy = fma(r.omegaThreeHalves, mxxMyy, dxux);
+    const R dzuz = fma(r.omegaThreeHalves, mxxMzz, dxux);
 
-    // cumulants back to central moments (:478-505)
-    // (the reference's (1/3) X / rho and (9 P + 3 S) / (9 rho) - drho / (9 rho)
-    // regrouped as X (1/(3 rho)) and P / rho + S / (3 rho) - drho / (9 rho))
-    const R oor3 = oneOverRho * cst<R>(1, 3);
-    const R dr9 = drho * oneOverRho * cst<R>(1, 9);
-    m211 = fma(fma(fma(R(3), m200, R(1)), m011, R(6) * (m110 * m101)), oor3, cm211);
-    m121 = fma(fma(fma(R(3), m020, R(1)), m101, R(6) * (m110 * m011)), oor3, cm121);
-    m112 = fma(fma(fma(R(3), m002, R(1)), m110, R(6) * (m101 * m011)), oor3, cm112);
-    m220 = fma(fma(m200, m020, R(2) * (m110 * m110)), oneOverRho, fma(m200 + m020, oor3, cm220 - dr9));
-    m202 = fma(fma(m200, m002, R(2) * (m101 * m101)), oneOverRho, fma(m200 + m002, oor3, cm202 - dr9));
-    m022 = fma(fma(m002, m020, R(2) * (m011 * m011)), oneOverRho, fma(m002 + m020, oor3, cm022 - dr9));
-    m122 = fma(fma(m002, m120, fma(m020, m102, fma(R(4) * m011, m111, R(2) * fma(m101, m021, m110 * m012)))),
-               oneOverRho, (m120 + m102) * oor3);
-    m212 = fma(fma(m002, m210, fma(m200, m012, fma(R(4) * m101, m111, R(2) * fma(m011, m201, m110 * m102)))),
-               oneOverRho, (m210 + m012) * oor3);
-    m221 = fma(fma(m200, m021, fma(m020, m201, fma(R(4) * m110, m111, R(2) * fma(m101, m120, m011 * m210)))),
-               oneOverRho, (m021 + m201) * oor3);
-    m222 = -c222Term(m111, m200, m020, m002, m022, m202, m220, m011, m101, m110, m211, m121, m112, m120, m102, m210,
-                     m012, m201, m021, oneOverRho, drho);
+    // second order relaxation with correction (:387-389).  p, q, s: halves of
+    // the post-collision c200, c020, c002 less rho / 3; their sum is trace
+    const R sx = vx2 * dxux, sy = vy2 * dyuy, sz = vz2 * dzuz;
+    const R trace = R(-0.75) * (sx + sy + sz);
+    const R xMy = fma(r.keepHalf, mxxMyy, r.corrHalf * (sx - sy));
+    const R xMz = fma(r.keepHalf, mxxMzz, r.corrHalf * (sx - sz));
+    const R p = cst<R>(1, 3) * (xMy + xMz + trace);
+    const R q = p - xMy;
+    const R s = p - xMz;
+    // mixed moments: post-collision a = c011 / 4, b = c101 / 4, c = c110 / 4;
+    // the linear part of the fourth-order mixed ones (c011 / 3 of the closure
+    // and the optimised equilibrium, :452-457, both multiples of the pre-collision c011)
+    const R a = r.keepQuarter * m011, b = r.keepQuarter * m101, c = r.keepQuarter * m110;
+    const R a4 = r.keep * m011, b4 = r.keep * m101, c4 = r.keep * m110;
+    const R la = r.mixed4 * m011, lb = r.mixed4 * m101, lc = r.mixed4 * m110;
+    const R mixed = fma(c, m110, fma(b, m101, a * m011));
 
-    // first moments change sign (force, :512-514)
-    m100 = -m100;
-    m010 = -m010;
-    m001 = -m001;
+    // third order with quartic limiters (:404-417), scaled: t4 = c111 / 2, the rest / 8
+    const R t4 = limitedMoment(m111, r.limD, r.qlD);
+    const R xxyP = limitedMoment(m210 + m012, r.limP, r.qlP), xxyM = limitedMoment(m210 - m012, r.limM, r.qlM);
+    const R xxzP = limitedMoment(m201 + m021, r.limP, r.qlP), xxzM = limitedMoment(m201 - m021, r.limM, r.qlM);
+    const R xyyP = limitedMoment(m120 + m102, r.limP, r.qlP), xyyM = limitedMoment(m120 - m102, r.limM, r.qlM);
+    m210 = xxyP + xxyM;
+    m012 = xxyP - xxyM;
+    m201 = xxzP + xxzM;
+    m021 = xxzP - xxzM;
+    m120 = xyyP + xyyM;
+    m102 = xyyP - xyyM;
 
-    // backward chimera, x then y then z (:525-557)
-    centralMomentsToPopulations(f, vvx, vvy, vvz);
+    // fourth order: Gaussian closure plus the modified equilibrium (:452-457, :478-488)
+    const R n211 = fma(b4, c, p * a), n121 = fma(a4, c, q * b), n112 = fma(a4, b, s * c);
+    const R n220 = fma(R(2) * c4, c, p * q), n202 = fma(R(2) * b4, b, p * s), n022 = fma(R(2) * a4, a, q * s);
+    const R divergence = dxux + dyuy + dzuz;
+    const R base = fma(r.fourthA4, divergence, fma(cst<R>(1, 6), trace, cst<R>(1, 36) * drho));
+    m220 = fma(n220, oneOverRho, fma(-cst<R>(1, 6), s, fma(r.minusFourthA4, dzuz, base)));
+    m202 = fma(n202, oneOverRho, fma(-cst<R>(1, 6), q, fma(r.minusFourthA4, dyuy, base)));
+    m022 = fma(n022, oneOverRho, fma(-cst<R>(1, 6), p, fma(r.minusFourthA4, dxux, base)));
+    m211 = fma(n211, oneOverRho, la);
+    m121 = fma(n121, oneOverRho, lb);
+    m112 = fma(n112, oneOverRho, lc);
+
+    // fifth and sixth order: cumulants zero (:463-471, :489-505)
+    {
+        const R third = cst<R>(1, 3);
+        const R n122 = fma(a4, t4, fma(b4, m021, fma(c4, m012, fma(q, m102, s * m120))));
+        const R n212 = fma(b4, t4, fma(a4, m201, fma(c4, m102, fma(p, m012, s * m210))));
+        const R n221 = fma(c4, t4, fma(b4, m120, fma(a4, m210, fma(q, m201, p * m021))));
+        m122 = fma(n122, oneOverRho, third * xyyP);
+        m212 = fma(n212, oneOverRho, third * xxyP);
+        m221 = fma(n221, oneOverRho, third * xxzP);
+        const R e = fma(m201, m021, fma(m210, m012, m120 * m102));
+        const R g = fma(divergence, trace, -fma(p, dxux, fma(q, dyuy, s * dzuz)));
+        const R first = fma(R(2), fma(R(2), e, t4 * t4),
+                            fma(cst<R>(1, 6), n220 + n202 + n022, fma(r.twoFourthB, mixed, r.fourthA4 * g)));
+        const R second = fma(R(2), fma(b4, n121, c4 * n112), p * n022);
+        m222 = fma(fma(second, oneOverRho, first), oneOverRho,
+                   fma(cst<R>(1, 6), base, r.fourthA24 * divergence));
+    }
+
+    // the remaining scaled moments; m000 = drho stays
+    const R drho6 = cst<R>(1, 6) * drho;
+    m200 = p + drho6;
+    m020 = q + drho6;
+    m002 = s + drho6;
+    m011 = a;
+    m101 = b;
+    m110 = c;
+    m111 = R(0.25) * t4;
+
+    scaledMomentsToPopulations(f, vvx, vvy, vvz);
 
     drho_out = drho;
     vx_out = vvx;

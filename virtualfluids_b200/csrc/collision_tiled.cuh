@@ -123,6 +123,7 @@ struct TiledArgs {
     uint32_t axisOff[3][2];
     K17Rates<R> rates;
     R fx, fy, fz, gfx, gfy, gfz, forceFactor;
+    bool forced; // (fx, fy, fz) is not zero
     // the same rates and forces duplicated into register pairs (paired kernel)
     K17Rates<F2> rates2;
     F2 fx2, fy2, fz2;
@@ -202,7 +203,7 @@ __device__ __forceinline__ void collideNode(const TiledArgs<S>& a, typename Stor
             a.bfz[k] = R(0);
         }
         R drho, ux, uy, uz;
-        k17Collide<R>(f, a.rates, fx, fy, fz, drho, ux, uy, uz);
+        k17Collide<R>(f, a.rates, fx, fy, fz, drho, ux, uy, uz, BF || a.forced);
         if (WM) {
             a.vx[k] = ux;
             a.vy[k] = uy;
@@ -460,7 +461,7 @@ __global__ void __launch_bounds__(C::T / 2, C::MINB) pairKernel(const TiledArgs<
     }
     F2 drho, ux, uy, uz;
     if constexpr (OP == Op::K17)
-        k17Collide<F2>(f, a.rates2, fx, fy, fz, drho, ux, uy, uz);
+        k17Collide<F2>(f, a.rates2, fx, fy, fz, drho, ux, uy, uz, BF || a.forced);
     else
         bgkCollide<F2>(f, a.rates2.omega);
     if (WM) {
@@ -792,6 +793,7 @@ static int launchTiled(Op op, const vfb_collision_plan_impl& p, const vfb_collis
     a.fx = a.gfx * R(0.5) * a.forceFactor;
     a.fy = a.gfy * R(0.5) * a.forceFactor;
     a.fz = a.gfz * R(0.5) * a.forceFactor;
+    a.forced = !(a.fx == R(0) && a.fy == R(0) && a.fz == R(0));
     if constexpr (sizeof(R) == 4) {
         a.rates2 = pairRates(a.rates);
         a.fx2 = F2(a.fx);

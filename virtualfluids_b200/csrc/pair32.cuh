@@ -56,9 +56,15 @@ __device__ __forceinline__ F2 fabs(F2 a) { return pairOf(make_float2(fabsf(a.v.x
 
 #ifdef __CUDA_ARCH__
 template <>
-__device__ __forceinline__ F2 limiterQuotient<F2>(F2 x, F2 y)
+__device__ __forceinline__ F2 limiterReciprocal<F2>(F2 x)
 {
-    return pairOf(make_float2(__fdividef(x.v.x, y.v.x), __fdividef(x.v.y, y.v.y)));
+    return F2(approximateReciprocal(x.v.x), approximateReciprocal(x.v.y));
+}
+template <>
+__device__ __forceinline__ F2 reciprocal<F2>(F2 x)
+{
+    const F2 r = limiterReciprocal(x);
+    return fma(fma(-x, r, F2(1.0f)), r, r);
 }
 #endif
 #endif
@@ -67,25 +73,9 @@ __device__ __forceinline__ F2 limiterQuotient<F2>(F2 x, F2 y)
 inline K17Rates<F2> pairRates(const K17Rates<float>& r)
 {
     K17Rates<F2> p;
-    p.omega = F2(r.omega);
-    p.OxyyPxzz = F2(r.OxyyPxzz);
-    p.OxyyMxzz = F2(r.OxyyMxzz);
-    p.Oxyz = F2(r.Oxyz);
-    p.oneMinusOxyyPxzz = F2(r.oneMinusOxyyPxzz);
-    p.oneMinusOxyyMxzz = F2(r.oneMinusOxyyMxzz);
-    p.oneMinusOxyz = F2(r.oneMinusOxyz);
-    p.factorA = F2(r.factorA);
-    p.factorB = F2(r.factorB);
-    p.minusTau = F2(r.minusTau);
-    p.halfMinusOmega = F2(r.halfMinusOmega);
-    p.omegaThreeHalves = F2(r.omegaThreeHalves);
-    p.minusThreeOmega = F2(r.minusThreeOmega);
-    p.secondOrderCorrection = F2(r.secondOrderCorrection);
-    p.qlP = F2(r.qlP);
-    p.qlM = F2(r.qlM);
-    p.qlD = F2(r.qlD);
-    p.fourthA = F2(r.fourthA);
-    p.fourthB = F2(r.fourthB);
+#define VFB_PAIR(name) p.name = F2(r.name);
+    VFB_K17_RATES(VFB_PAIR)
+#undef VFB_PAIR
     return p;
 }
 

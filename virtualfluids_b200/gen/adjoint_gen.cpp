@@ -33,7 +33,7 @@
 
 namespace vfgen
 {
-enum Op { INPUT, PARAM, CONST, ADD, SUB, MUL, DIV, FDIV, NEG, FMA, ABS };
+enum Op { INPUT, PARAM, CONST, ADD, SUB, MUL, RCP, FRCP, NEG, FMA, ABS };
 
 struct Node {
     Op op;
@@ -86,8 +86,8 @@ inline Sym make(Op op, const Sym& a, const Sym& b = Sym(), const Sym& c = Sym())
             case ADD: r = fx + fy; break;
             case SUB: r = fx - fy; break;
             case MUL: r = fx * fy; break;
-            case DIV:
-            case FDIV: r = fx / fy; break;
+            case RCP:
+            case FRCP: r = 1.0f / fx; break;
             case NEG: r = -fx; break;
             case FMA: r = std::fmaf(fx, fy, fz); break;
             case ABS: r = std::fabs(fx); break;
@@ -98,8 +98,8 @@ inline Sym make(Op op, const Sym& a, const Sym& b = Sym(), const Sym& c = Sym())
             case ADD: r = x + y; break;
             case SUB: r = x - y; break;
             case MUL: r = x * y; break;
-            case DIV:
-            case FDIV: r = x / y; break;
+            case RCP:
+            case FRCP: r = 1.0 / x; break;
             case NEG: r = -x; break;
             case FMA: r = std::fma(x, y, z); break;
             case ABS: r = std::fabs(x); break;
@@ -119,7 +119,13 @@ inline Sym make(Op op, const Sym& a, const Sym& b = Sym(), const Sym& c = Sym())
 inline Sym operator+(const Sym& a, const Sym& b) { return make(ADD, a, b); }
 inline Sym operator-(const Sym& a, const Sym& b) { return make(SUB, a, b); }
 inline Sym operator*(const Sym& a, const Sym& b) { return make(MUL, a, b); }
-inline Sym operator/(const Sym& a, const Sym& b) { return make(DIV, a, b); }
+// constants only (the operator divides through reciprocal / limiterReciprocal)
+inline Sym operator/(const Sym& a, const Sym& b)
+{
+    if (!isConst(a) || !isConst(b))
+        std::abort();
+    return tape->single ? Sym((double)((float)cval(a) / (float)cval(b))) : Sym(cval(a) / cval(b));
+}
 inline Sym operator-(const Sym& a) { return make(NEG, a); }
 inline Sym& operator+=(Sym& a, const Sym& b) { return a = a + b; }
 inline Sym& operator-=(Sym& a, const Sym& b) { return a = a - b; }
@@ -151,9 +157,14 @@ struct SymF : vfgen::Sym {
     SymF(const vfgen::Sym& s) : Sym(s) {}
 };
 template <>
-__host__ __device__ inline vfgen::Sym limiterQuotient<vfgen::Sym>(vfgen::Sym x, vfgen::Sym y)
+__host__ __device__ inline vfgen::Sym reciprocal<vfgen::Sym>(vfgen::Sym x)
 {
-    return vfgen::make(vfgen::FDIV, x, y);
+    return vfgen::make(vfgen::RCP, x);
+}
+template <>
+__host__ __device__ inline vfgen::Sym limiterReciprocal<vfgen::Sym>(vfgen::Sym x)
+{
+    return vfgen::make(vfgen::FRCP, x);
 }
 } // namespace vfb
 
@@ -212,8 +223,8 @@ struct Emitter {
         case ADD: return val(n.a) + " + " + val(n.b);
         case SUB: return val(n.a) + " - " + val(n.b);
         case MUL: return val(n.a) + " * " + val(n.b);
-        case DIV: return val(n.a) + " / " + val(n.b);
-        case FDIV: return "limiterQuotient<R>(" + val(n.a) + ", " + val(n.b) + ")";
+        case RCP: return "reciprocal<R>(" + val(n.a) + ")";
+        case FRCP: return "limiterReciprocal<R>(" + val(n.a) + ")";
         case NEG: return "-" + val(n.a);
         case FMA: return "fma(" + val(n.a) + ", " + val(n.b) + ", " + val(n.c) + ")";
         case ABS: return "fabs(" + val(n.a) + ")";
@@ -288,15 +299,10 @@ struct Emitter {
                 acc(n.a, g + " * " + val(n.b), false);
                 acc(n.b, g + " * " + val(n.a), false);
                 break;
-            case DIV:
-            case FDIV: {
-                // q = a / b: dq/da = 1/b, dq/db = -q/b
-                const std::string s = "s" + std::to_string(i);
-                std::fprintf(out, "    const R %s = %s / %s;\n", s.c_str(), g.c_str(), val(n.b).c_str());
-                acc(n.a, s, false);
-                acc(n.b, s + " * " + val(i), true);
+            case RCP:
+            case FRCP: // d(1/a) = -(1/a)^2 da
+                acc(n.a, g + " * " + val(i) + " * " + val(i), true);
                 break;
-            }
             case NEG: acc(n.a, g, true); break;
             case FMA:
                 acc(n.a, g + " * " + val(n.b), false);
@@ -335,15 +341,9 @@ void traceK17(Tape& tp, bool single, Emitter& em)
         em.inputIds.push_back(f[d].id);
     }
     vfb::K17Rates<R> r;
-    const char* names[] = { "r.omega", "r.OxyyPxzz", "r.OxyyMxzz", "r.Oxyz", "r.oneMinusOxyyPxzz",
-                            "r.oneMinusOxyyMxzz", "r.oneMinusOxyz", "r.factorA", "r.factorB", "r.minusTau",
-                            "r.halfMinusOmega", "r.omegaThreeHalves", "r.minusThreeOmega",
-                            "r.secondOrderCorrection", "r.qlP", "r.qlM", "r.qlD", "r.fourthA", "r.fourthB" };
-    R* fields[] = { &r.omega, &r.OxyyPxzz, &r.OxyyMxzz, &r.Oxyz, &r.oneMinusOxyyPxzz, &r.oneMinusOxyyMxzz,
-                    &r.oneMinusOxyz, &r.factorA, &r.factorB, &r.minusTau, &r.halfMinusOmega, &r.omegaThreeHalves,
-                    &r.minusThreeOmega, &r.secondOrderCorrection, &r.qlP, &r.qlM, &r.qlD, &r.fourthA, &r.fourthB };
-    for (size_t i = 0; i < sizeof(fields) / sizeof(fields[0]); ++i)
-        *fields[i] = input(names[i], PARAM);
+#define VFB_INPUT(name) r.name = input("r." #name, PARAM);
+    VFB_K17_RATES(VFB_INPUT)
+#undef VFB_INPUT
     R fx = input("fx", PARAM), fy = input("fy", PARAM), fz = input("fz", PARAM);
     em.forceIds = { fx.id, fy.id, fz.id };
     R drho, vx, vy, vz;
@@ -368,16 +368,24 @@ namespace vfb
 inline SymF operator+(const SymF& a, const SymF& b) { return vfgen::make(vfgen::ADD, a, b); }
 inline SymF operator-(const SymF& a, const SymF& b) { return vfgen::make(vfgen::SUB, a, b); }
 inline SymF operator*(const SymF& a, const SymF& b) { return vfgen::make(vfgen::MUL, a, b); }
-inline SymF operator/(const SymF& a, const SymF& b) { return vfgen::make(vfgen::DIV, a, b); }
+inline SymF operator/(const SymF& a, const SymF& b)
+{
+    return static_cast<const vfgen::Sym&>(a) / static_cast<const vfgen::Sym&>(b);
+}
 inline SymF operator-(const SymF& a) { return vfgen::make(vfgen::NEG, a); }
 inline SymF& operator+=(SymF& a, const SymF& b) { return a = a + b; }
 inline SymF& operator-=(SymF& a, const SymF& b) { return a = a - b; }
 inline SymF fma(const SymF& a, const SymF& b, const SymF& c) { return vfgen::make(vfgen::FMA, a, b, c); }
 inline SymF fabs(const SymF& a) { return vfgen::make(vfgen::ABS, a); }
 template <>
-__host__ __device__ inline SymF limiterQuotient<SymF>(SymF x, SymF y)
+__host__ __device__ inline SymF reciprocal<SymF>(SymF x)
 {
-    return vfgen::make(vfgen::FDIV, x, y);
+    return vfgen::make(vfgen::RCP, x);
+}
+template <>
+__host__ __device__ inline SymF limiterReciprocal<SymF>(SymF x)
+{
+    return vfgen::make(vfgen::FRCP, x);
 }
 } // namespace vfb
 
