@@ -199,6 +199,7 @@ __device__ __forceinline__ void postBCEntry(R* __restrict__ dist, const BcLattic
     R drho, vx1, vx2, vx3;
     bcMacros(g, drho, vx1, vx2, vx3);
     const R cuSq = R(3) / R(2) * (vx1 * vx1 + vx2 * vx2 + vx3 * vx3) * (R(1) + drho);
+    const LinkRates<R> rates(lat.omega);
     R UX = R(0), UY = R(0), UZ = R(0);
     if (KIND == VFB_BC_VELOCITY_INTERPOLATED) {
         UX = __ldg(Vx + i);
@@ -220,8 +221,8 @@ __device__ __forceinline__ void postBCEntry(R* __restrict__ dist, const BcLattic
         const R w = weight<R>(d);
         const R feq = feqBC(drho, cdot<R>(d, vx1, vx2, vx3), cuSq, w);
         const R value = KIND == VFB_BC_VELOCITY_INTERPOLATED
-                            ? interpVelocity(qd, g[d], g[e], feq, lat.omega, cdot<R>(d, UX, UY, UZ), w)
-                            : interpNoSlip(qd, g[d], g[e], feq, lat.omega);
+                            ? interpVelocity(qd, g[d], g[e], feq, rates, cdot<R>(d, UX, UY, UZ), w)
+                            : interpNoSlip(qd, g[d], g[e], feq, rates);
         dist[cell<R>(slot<!EVEN>(e), N, L.k[loc(e)])] = value;
     }
 }
@@ -309,8 +310,9 @@ __device__ __forceinline__ void postScatterEntry(R* __restrict__ lam, const BcLa
         const int e = inv(d);
         const R t = tmp[(unsigned long long)d * n + i];
         const R w = weight<R>(d);
-        const R A = (R(1) - qd) / (R(1) + qd);
-        const R b = qd / (R(1) + qd);
+        const R r = linkReciprocal(R(1) + qd);
+        const R A = (R(1) - qd) * r;
+        const R b = qd * r;
         gg[d] += t * (A * R(0.5) * (R(1) + c1) + b);
         gg[e] += t * (A * R(0.5) * (c1 - R(1)) + b);
         const R gfeq = -t * A * omega * c1;
@@ -322,7 +324,7 @@ __device__ __forceinline__ void postScatterEntry(R* __restrict__ lam, const BcLa
         guz += gvel * R(cz(d));
         gcuSq -= gfeq * w;
         if (KIND == VFB_BC_VELOCITY_INTERPOLATED) {
-            const R gU = -t * R(6) * w / (R(1) + qd);
+            const R gU = -t * R(6) * w * r;
             gUx += gU * R(cx(d));
             gUy += gU * R(cy(d));
             gUz += gU * R(cz(d));
@@ -446,32 +448,7 @@ __global__ void __launch_bounds__(kThreads)
         for (int d = 0; d < 27; ++d)
             rec[(unsigned long long)d * n + i] = f[d];
     }
-    // the arithmetic of bcPressureKernel (bc.cu), operation for operation
-    R drho1 = pyramidDensity(f);
-    const R oneOverRho = R(1) / (drho1 + R(1));
-    const R vx1 = pyramidJx(f) * oneOverRho;
-    const R vx2 = pyramidJy(f) * oneOverRho;
-    const R vx3 = pyramidJz(f) * oneOverRho;
-    const R cusq = R(3) / R(2) * (vx1 * vx1 + vx2 * vx2 + vx3 * vx3);
-#pragma unroll
-    for (int d = 0; d < 27; ++d) {
-        if (d == d000) {
-            f[d] -= R(8) / R(27) * (drho1 - (drho1 + R(1)) * cusq);
-        } else {
-            const R cu = cdot<R>(d, vx1, vx2, vx3);
-            f[d] -= weight<R>(d) * (drho1 + (drho1 + R(1)) * (R(3) * cu + R(9) / R(2) * cu * cu - cusq));
-        }
-    }
-    drho1 = __ldg(rhoBC + i);
-#pragma unroll
-    for (int d = 0; d < 27; ++d) {
-        if (d == d000) {
-            f[d] += R(8) / R(27) * (drho1 - (drho1 + R(1)) * cusq);
-        } else {
-            const R cu = cdot<R>(d, vx1, vx2, vx3);
-            f[d] += weight<R>(d) * (drho1 + (drho1 + R(1)) * (R(3) * cu + R(9) / R(2) * cu * cu - cusq));
-        }
-    }
+    pressureShift(f, __ldg(rhoBC + i));
 #pragma unroll
     for (int d = 0; d < 27; ++d) {
         const int c = axis == 0 ? cx(d) : axis == 1 ? cy(d) : cz(d);

@@ -73,11 +73,18 @@ __global__ void bcLocationsKernel(const int32_t* __restrict__ bcK, uint32_t n, c
         out[(unsigned long long)l * n + i] = L.k[l];
 }
 
-// six resident blocks of 128 threads: the gathers of a wall entry are DRAM
-// bursts, so more of them in flight matter more than the few registers the
-// 80-register bound spills
+// Resident blocks of 128 threads the registers are sized for.  FP32
+// arithmetic: six, since the gathers of a wall entry are DRAM bursts, and more
+// of them in flight matter more than the few registers the 80-register bound
+// spills.  FP64: three (168 registers); at six the 53 values an entry holds
+// spilled 240 to 400 bytes a thread.
+template <class R>
+constexpr int bcBlocks()
+{
+    return sizeof(R) == 8 ? 3 : 6;
+}
 template <class S, int KIND, bool EVEN>
-__global__ void __launch_bounds__(128, 6) bcPostKernel(S* __restrict__ dist, const BcLattice<typename Storage<S>::R> lat,
+__global__ void __launch_bounds__(128, bcBlocks<typename Storage<S>::R>()) bcPostKernel(S* __restrict__ dist, const BcLattice<typename Storage<S>::R> lat,
                                                      const int32_t* __restrict__ bcK,
                                                      const typename Storage<S>::R* __restrict__ q, uint32_t nBC,
                                                      const typename Storage<S>::R* __restrict__ Vx,
@@ -95,8 +102,9 @@ __global__ void __launch_bounds__(128, 6) bcPostKernel(S* __restrict__ dist, con
 
 // PressureNonEquilibriumCompressible.cu:75-309: the neighbour's
 // pre-collision populations with their equilibrium part moved from the
-// neighbour's density to the prescribed one, written into the BC node's
-// directions whose component along the normal axis differs from the normal's
+// neighbour's density to the prescribed one (pressureShift), written into the
+// BC node's directions whose component along the normal axis differs from the
+// normal's
 template <class S, bool EVEN>
 __global__ void __launch_bounds__(128) bcPressureKernel(S* __restrict__ dist, const BcLattice<typename Storage<S>::R> lat,
                                                          const int32_t* __restrict__ bcK,
@@ -127,31 +135,7 @@ __global__ void __launch_bounds__(128) bcPressureKernel(S* __restrict__ dist, co
 #pragma unroll
     for (int d = 0; d < 27; ++d)
         f[d] = Storage<S>::load(dist + (unsigned long long)slot<EVEN>(d) * N + LN.k[loc(d)], d);
-    R drho1 = pyramidDensity(f);
-    const R oneOverRho = R(1) / (drho1 + R(1));
-    const R vx1 = pyramidJx(f) * oneOverRho;
-    const R vx2 = pyramidJy(f) * oneOverRho;
-    const R vx3 = pyramidJz(f) * oneOverRho;
-    const R cusq = R(3) / R(2) * (vx1 * vx1 + vx2 * vx2 + vx3 * vx3);
-#pragma unroll
-    for (int d = 0; d < 27; ++d) {
-        if (d == d000) {
-            f[d] -= R(8) / R(27) * (drho1 - (drho1 + R(1)) * cusq);
-        } else {
-            const R cu = cdot<R>(d, vx1, vx2, vx3);
-            f[d] -= weight<R>(d) * (drho1 + (drho1 + R(1)) * (R(3) * cu + R(9) / R(2) * cu * cu - cusq));
-        }
-    }
-    drho1 = __ldg(rhoBC + i);
-#pragma unroll
-    for (int d = 0; d < 27; ++d) {
-        if (d == d000) {
-            f[d] += R(8) / R(27) * (drho1 - (drho1 + R(1)) * cusq);
-        } else {
-            const R cu = cdot<R>(d, vx1, vx2, vx3);
-            f[d] += weight<R>(d) * (drho1 + (drho1 + R(1)) * (R(3) * cu + R(9) / R(2) * cu * cu - cusq));
-        }
-    }
+    pressureShift(f, __ldg(rhoBC + i));
 #pragma unroll
     for (int d = 0; d < 27; ++d) {
         const int c = axis == 0 ? cx(d) : axis == 1 ? cy(d) : cz(d);

@@ -57,6 +57,7 @@ __device__ __forceinline__ void bcPostEntry(S* __restrict__ dist, unsigned long 
     }
     // slip: normal components are removed for each axis with an active axis direction
     bool flagX = false, flagY = false, flagZ = false;
+    const LinkRates<R> rates(omega);
     // all q values first, so that their loads are in flight together instead
     // of one per direction behind the branch on the previous one
     R qv[26];
@@ -81,13 +82,13 @@ __device__ __forceinline__ void bcPostEntry(S* __restrict__ dist, unsigned long 
             value = g[d] + k6 * cdot<R>(e, UX, UY, UZ);
         } else if (KIND == VFB_BC_NOSLIP_INTERPOLATED) {
             const R feq = feqBC(drho, cdot<R>(d, vx1, vx2, vx3), cuSq, w);
-            value = interpNoSlip(qd, g[d], g[e], feq, omega);
+            value = interpNoSlip(qd, g[d], g[e], feq, rates);
         } else if (KIND == VFB_BC_VELOCITY_INTERPOLATED) {
             const R feq = feqBC(drho, cdot<R>(d, vx1, vx2, vx3), cuSq, w);
-            value = interpVelocity(qd, g[d], g[e], feq, omega, cdot<R>(d, UX, UY, UZ), w);
+            value = interpVelocity(qd, g[d], g[e], feq, rates, cdot<R>(d, UX, UY, UZ), w);
         } else if (KIND == VFB_BC_VELOCITY_WITH_PRESSURE) {
             const R feq = feqBC(drho, cdot<R>(d, vx1, vx2, vx3), cuSq, w);
-            value = interpVelocity(qd, g[d], g[e], feq, omega, cdot<R>(d, UX, UY, UZ), w) - w * drho;
+            value = interpVelocity(qd, g[d], g[e], feq, rates, cdot<R>(d, UX, UY, UZ), w) - w * drho;
         } else {
             if (order(d) == 1) {
                 if (cx(d) != 0)
@@ -99,7 +100,7 @@ __device__ __forceinline__ void bcPostEntry(S* __restrict__ dist, unsigned long 
             }
             const R sx = flagX ? R(0) : vx1, sy = flagY ? R(0) : vx2, sz = flagZ ? R(0) : vx3;
             const R feq = feqBC(drho, cdot<R>(d, vx1, vx2, vx3), cuSq, w);
-            value = interpVelocity(qd, g[d], g[e], feq, omega, cdot<R>(d, sx, sy, sz), w);
+            value = interpVelocity(qd, g[d], g[e], feq, rates, cdot<R>(d, sx, sy, sz), w);
         }
         Storage<S>::store(target, value, d);
     }

@@ -1,13 +1,14 @@
 // bc_math.cuh -- per-node formulas of the post-collision boundary conditions,
 // shared by the BC kernels (bc.cu) and their adjoints (adjoint.cu) so that
 // both run the same arithmetic.  Formulas: KernelUtilities.h:171-195 and the
-// plain macroscopic sums of NoSlipInterpolatedCompressible.cu:144-160.
+// macroscopic sums of NoSlipInterpolatedCompressible.cu:144-160.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
+#include "collision_math.cuh"
 #include "d3q27.cuh"
 
 namespace vfb
@@ -30,52 +31,31 @@ struct BcLattice {
     R omega;
 };
 
-// drho and velocity from post-collision populations with the plain sums of
-// NoSlipInterpolatedCompressible.cu:144-160 (g[d] moves in direction d)
+// drho and velocity from post-collision populations (g[d] moves in direction
+// d): the sums of NoSlipInterpolatedCompressible.cu:144-160 as trees, since a
+// short list's launch lasts as long as one entry's dependent chain
 template <class R>
 __device__ __forceinline__ void bcMacros(const R* g, R& drho, R& vx1, R& vx2, R& vx3)
 {
-    R s = g[dPMP];
-    s = s + g[dMPP];
-    s = s + g[dPPP];
-    s = s + g[dMMP];
-    s = s + g[dPMM];
-    s = s + g[dMPM];
-    s = s + g[dPPM];
-    s = s + g[dMMM];
-    s = s + g[d0PM];
-    s = s + g[d0MP];
-    s = s + g[d0PP];
-    s = s + g[d0MM];
-    s = s + g[dP0M];
-    s = s + g[dM0P];
-    s = s + g[dP0P];
-    s = s + g[dM0M];
-    s = s + g[dPM0];
-    s = s + g[dMP0];
-    s = s + g[dPP0];
-    s = s + g[dMM0];
-    s = s + g[d00P];
-    s = s + g[d00M];
-    s = s + g[d0P0];
-    s = s + g[d0M0];
-    s = s + g[dP00];
-    s = s + g[dM00];
-    s = s + g[d000];
-    drho = s;
-    const R r1 = R(1) + s;
-    vx1 = (((g[dPMP] - g[dMPM]) - (g[dMPP] - g[dPMM])) + ((g[dPPP] - g[dMMM]) - (g[dMMP] - g[dPPM])) +
-           ((g[dP0M] - g[dM0P]) + (g[dP0P] - g[dM0M])) + ((g[dPM0] - g[dMP0]) + (g[dPP0] - g[dMM0])) +
-           (g[dP00] - g[dM00])) /
-          r1;
-    vx2 = ((-(g[dPMP] - g[dMPM]) + (g[dMPP] - g[dPMM])) + ((g[dPPP] - g[dMMM]) - (g[dMMP] - g[dPPM])) +
-           ((g[d0PM] - g[d0MP]) + (g[d0PP] - g[d0MM])) + (-(g[dPM0] - g[dMP0]) + (g[dPP0] - g[dMM0])) +
-           (g[d0P0] - g[d0M0])) /
-          r1;
-    vx3 = (((g[dPMP] - g[dMPM]) + (g[dMPP] - g[dPMM])) + ((g[dPPP] - g[dMMM]) + (g[dMMP] - g[dPPM])) +
-           (-(g[d0PM] - g[d0MP]) + (g[d0PP] - g[d0MM])) + ((g[dP0P] - g[dM0M]) - (g[dP0M] - g[dM0P])) +
-           (g[d00P] - g[d00M])) /
-          r1;
+    drho = pyramidDensity(g);
+    const R oneOverRho = reciprocal(R(1) + drho);
+    vx1 = pyramidJx(g) * oneOverRho;
+    vx2 = pyramidJy(g) * oneOverRho;
+    vx3 = pyramidJz(g) * oneOverRho;
+}
+
+// 1 / (1 + q) of a link, q in [0, 1]: in FP64 the single-precision reciprocal
+// and two Newton-Raphson steps r (2 - x r), instead of a division per link
+__device__ __forceinline__ float linkReciprocal(float x) { return reciprocal(x); }
+__device__ __forceinline__ double linkReciprocal(double x)
+{
+#ifdef __CUDA_ARCH__
+    double r = (double)approximateReciprocal((float)x);
+    r = fma(fma(-x, r, 1.0), r, r);
+    return fma(fma(-x, r, 1.0), r, r);
+#else
+    return 1.0 / x;
+#endif
 }
 
 // KernelUtilities.h:171-174
@@ -85,27 +65,66 @@ __device__ __forceinline__ R feqBC(R drho, R vel, R cuSq, R w)
     return w * (drho + R(9) / R(2) * vel * vel * (R(1) + drho) - cuSq);
 }
 
-// KernelUtilities.h:189-195
+// The relaxation of the interpolated links: 2 omega and 1 / (1 - omega)
 template <class R>
-__device__ __forceinline__ R interpNoSlip(R q, R f, R finv, R feq, R omega)
+struct LinkRates {
+    R twoOmega, inverse;
+    __device__ __forceinline__ explicit LinkRates(R omega) : twoOmega(R(2) * omega), inverse(R(1) / (R(1) - omega)) {}
+};
+
+// KernelUtilities.h:176-195: the interpolated bounce-back of a link with wall
+// distance q, over the common denominator 1 + q (one reciprocal a link, where
+// the formula as written has three divisions; those were most of an FP64
+// list's time, and the chain that a short list waits for):
+//   [ (1 - q) / 2 (f - finv + (f + finv - 2 omega feq) / (1 - omega)) + q (f + finv) - moving ] / (1 + q)
+// moving: 6 w c.u of a moving wall, 0 of one at rest
+template <class R>
+__device__ __forceinline__ R interpolatedLink(R q, R f, R finv, R feq, const LinkRates<R>& r, R moving)
 {
-    return (R(1) - q) / (R(1) + q) * (f - finv + (f + finv - R(2) * feq * omega) / (R(1) - omega)) * (R(1) / R(2)) +
-           (q * (f + finv)) / (R(1) + q);
+    const R s = f + finv;
+    const R t = fma(fma(-r.twoOmega, feq, s), r.inverse, f - finv);
+    return fma(fma(R(-0.5), q, R(0.5)), t, fma(q, s, -moving)) * linkReciprocal(R(1) + q);
 }
 
-// KernelUtilities.h:176-182
 template <class R>
-__device__ __forceinline__ R interpVelocity(R q, R f, R finv, R feq, R omega, R vel, R w)
+__device__ __forceinline__ R interpNoSlip(R q, R f, R finv, R feq, const LinkRates<R>& r)
 {
-    return (R(1) - q) / (R(1) + q) * (f - finv + (f + finv - R(2) * feq * omega) / (R(1) - omega)) * (R(1) / R(2)) +
-           (q * (f + finv) - R(6) * w * vel) / (R(1) + q);
+    return interpolatedLink(q, f, finv, feq, r, R(0));
+}
+
+template <class R>
+__device__ __forceinline__ R interpVelocity(R q, R f, R finv, R feq, const LinkRates<R>& r, R vel, R w)
+{
+    return interpolatedLink(q, f, finv, feq, r, R(6) * w * vel);
 }
 
 // KernelUtilities.h:199-206 (the interpolated no-slip value minus w drho)
 template <class R>
-__device__ __forceinline__ R interpNoSlipPressure(R q, R f, R finv, R feq, R omega, R drho, R w)
+__device__ __forceinline__ R interpNoSlipPressure(R q, R f, R finv, R feq, const LinkRates<R>& r, R drho, R w)
 {
-    return interpNoSlip(q, f, finv, feq, omega) - w * drho;
+    return interpNoSlip(q, f, finv, feq, r) - w * drho;
+}
+
+// PressureNonEquilibriumCompressible.cu:75-309: populations f of the
+// neighbour with their equilibrium moved from its density to 1 + drhoBC at the
+// same velocity: f_d + w_d (drhoBC - drho) (1 + 3 c.u + 9/2 (c.u)^2 - 3/2 u^2),
+// the reference's subtraction and addition of two equilibria in one term
+template <class R>
+__device__ __forceinline__ void pressureShift(R* f, R drhoBC)
+{
+    const R drho = pyramidDensity(f);
+    const R oneOverRho = reciprocal(drho + R(1));
+    const R vx1 = pyramidJx(f) * oneOverRho;
+    const R vx2 = pyramidJy(f) * oneOverRho;
+    const R vx3 = pyramidJz(f) * oneOverRho;
+    const R keep = R(1) - R(3) / R(2) * (vx1 * vx1 + vx2 * vx2 + vx3 * vx3);
+    const R delta = drhoBC - drho;
+    f[d000] = fma(R(8) / R(27) * delta, keep, f[d000]);
+#pragma unroll
+    for (int d = 1; d < 27; ++d) {
+        const R cu = cdot<R>(d, vx1, vx2, vx3);
+        f[d] = fma(weight<R>(d) * delta, fma(fma(R(9) / R(2), cu, R(3)), cu, keep), f[d]);
+    }
 }
 
 // The wall model's clip (iMEM.cuh:131-136): -3 F forceFactor formed in

@@ -94,6 +94,8 @@ __global__ void __launch_bounds__(128) bcStressKernel(S* __restrict__ dist, cons
         om = lat.omega / (R(1) + R(3) * lat.omega * fmax(R(0), nu));
     }
 
+    const LinkRates<R> rates(om);
+
     // 2. incoming populations of a wall at rest and the exchanged momentum
     R fin[26];
     R mom[3] = { R(0), R(0), R(0) };
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(128) bcStressKernel(S* __restrict__ dist, cons
         } else {
             const R feq = feqBC(drho, cdot<R>(d, vx1, vx2, vx3), cuSq, w);
             const R wp = d == dPP0 ? R(2) / R(27) : w;
-            fin[j] = interpNoSlipPressure(qv[j], g[d], g[inv(d)], feq, om, drho, wp);
+            fin[j] = interpNoSlipPressure(qv[j], g[d], g[inv(d)], feq, rates, drho, wp);
         }
         const R t = g[d] + fin[j];
         if (cx(d) > 0) mom[0] = mom[0] + t; else if (cx(d) < 0) mom[0] = mom[0] - t;
@@ -147,7 +149,7 @@ __global__ void __launch_bounds__(128) bcStressKernel(S* __restrict__ dist, cons
         const int e = inv(d);
         R term = R(6) * weight<R>(d) * cdot<R>(d, V[0], V[1], V[2]);
         if (KIND == VFB_BC_STRESS_INTERPOLATED)
-            term = term / (R(1) + qv[j]);
+            term = term * linkReciprocal(R(1) + qv[j]);
         Storage<S>::store(dist + (unsigned long long)slot<!EVEN>(e) * N + L.k[loc(e)], fin[j] - term, d);
         if (cx(d) > 0) mom[0] = mom[0] - term; else if (cx(d) < 0) mom[0] = mom[0] + term;
         if (cy(d) > 0) mom[1] = mom[1] - term; else if (cy(d) < 0) mom[1] = mom[1] + term;
