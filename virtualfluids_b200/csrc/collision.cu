@@ -15,6 +15,7 @@
 
 #include "capi_common.cuh"
 #include "collision_math.cuh"
+#include "collision_math16.cuh"
 #include "d3q27.cuh"
 #include "storage.cuh"
 #include "pdl.cuh"
@@ -35,7 +36,7 @@ struct CollisionKernelArgs {
     uint32_t nFluid;
     // the list's location table (8 * nFluid, vfb_bc_locations layout) or null
     const uint32_t* __restrict__ table;
-    K17Rates<R> rates;
+    typename K17Of<S>::template Rates<R> rates;
     R fx, fy, fz;         // forces * 1/2 * forceFactor
     bool forced;          // (fx, fy, fz) is not zero
     R gfx, gfy, gfz;      // raw global forces (body-force template)
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(kCollisionThreads) k17Kernel(const CollisionKe
     for (int d = 0; d < 27; ++d)
         f[d] = Storage<S>::load(a.base[d] + L.k[loc(d)], d);
     R drho, ux, uy, uz;
-    k17Collide<R>(f, a.rates, fx, fy, fz, drho, ux, uy, uz, BODY_FORCE || a.forced);
+    K17Of<S>::template collide<R>(f, a.rates, fx, fy, fz, drho, ux, uy, uz, BODY_FORCE || a.forced);
     if (WRITE_MACRO) {
         a.vx[k] = ux;
         a.vy[k] = uy;
@@ -394,8 +395,8 @@ static int launchCollision(bool bgk, const vfb_collision_args* a, cudaStream_t s
     k.nZ = a->neighborZ;
     k.fluid = a->fluidNodeIndices;
     k.nFluid = a->numberOfFluidNodes;
-    k.rates = makeK17Rates<R>((R)a->omega, (R)a->quadricLimiters[0], (R)a->quadricLimiters[1],
-                              (R)a->quadricLimiters[2]);
+    k.rates = K17Of<S>::template make<R>((R)a->omega, (R)a->quadricLimiters[0], (R)a->quadricLimiters[1],
+                                         (R)a->quadricLimiters[2]);
     k.forceFactor = (R)a->forceFactor;
     k.gfx = (R)a->forces[0];
     k.gfy = (R)a->forces[1];

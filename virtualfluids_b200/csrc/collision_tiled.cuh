@@ -44,6 +44,7 @@
 #include "bc_entry.cuh"
 #include "capi_common.cuh"
 #include "collision_math.cuh"
+#include "collision_math16.cuh"
 #include "d3q27.cuh"
 #include "storage.cuh"
 #include "pair32.cuh"
@@ -121,11 +122,11 @@ struct TiledArgs {
     // offset of the periodic image for a node that wraps on that axis}, both
     // modulo 2^32 (node index + offset is the location's index in [0, N))
     uint32_t axisOff[3][2];
-    K17Rates<R> rates;
+    typename K17Of<S>::template Rates<R> rates;
     R fx, fy, fz, gfx, gfy, gfz, forceFactor;
     bool forced; // (fx, fy, fz) is not zero
     // the same rates and forces duplicated into register pairs (paired kernel)
-    K17Rates<F2> rates2;
+    typename K17Of<S>::template Rates<F2> rates2;
     F2 fx2, fy2, fz2;
     R* rho;
     R* vx;
@@ -203,7 +204,7 @@ __device__ __forceinline__ void collideNode(const TiledArgs<S>& a, typename Stor
             a.bfz[k] = R(0);
         }
         R drho, ux, uy, uz;
-        k17Collide<R>(f, a.rates, fx, fy, fz, drho, ux, uy, uz, BF || a.forced);
+        K17Of<S>::template collide<R>(f, a.rates, fx, fy, fz, drho, ux, uy, uz, BF || a.forced);
         if (WM) {
             a.vx[k] = ux;
             a.vy[k] = uy;
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(C::T / 2, C::MINB) pairKernel(const TiledArgs<
     }
     F2 drho, ux, uy, uz;
     if constexpr (OP == Op::K17)
-        k17Collide<F2>(f, a.rates2, fx, fy, fz, drho, ux, uy, uz, BF || a.forced);
+        K17Of<S>::template collide<F2>(f, a.rates2, fx, fy, fz, drho, ux, uy, uz, BF || a.forced);
     else
         bgkCollide<F2>(f, a.rates2.omega);
     if (WM) {
@@ -784,8 +785,8 @@ static int launchTiled(Op op, const vfb_collision_plan_impl& p, const vfb_collis
         a.axisOff[ax][0] = strides[ax];
         a.axisOff[ax][1] = (uint32_t)(p.wrapDelta[ax] + (long long)strides[ax]);
     }
-    a.rates = makeK17Rates<R>((R)c->omega, (R)c->quadricLimiters[0], (R)c->quadricLimiters[1],
-                              (R)c->quadricLimiters[2]);
+    a.rates = K17Of<S>::template make<R>((R)c->omega, (R)c->quadricLimiters[0], (R)c->quadricLimiters[1],
+                                         (R)c->quadricLimiters[2]);
     a.forceFactor = (R)c->forceFactor;
     a.gfx = (R)c->forces[0];
     a.gfy = (R)c->forces[1];

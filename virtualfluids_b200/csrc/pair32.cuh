@@ -11,7 +11,7 @@
 
 #include <cuda_runtime.h>
 
-#include "collision_math.cuh"
+#include "collision_math16.cuh"
 
 namespace vfb
 {
@@ -69,12 +69,29 @@ __device__ __forceinline__ F2 reciprocal<F2>(F2 x)
 #endif
 #endif
 
+#ifdef __CUDA_ARCH__
+template <>
+__device__ __forceinline__ F2 termwise::limiterQuotient<F2>(F2 x, F2 y)
+{
+    return F2(__fdividef(x.v.x, y.v.x), __fdividef(x.v.y, y.v.y));
+}
+#endif
+
 // K17 rates of a launch duplicated into both halves
 inline K17Rates<F2> pairRates(const K17Rates<float>& r)
 {
     K17Rates<F2> p;
 #define VFB_PAIR(name) p.name = F2(r.name);
     VFB_K17_RATES(VFB_PAIR)
+#undef VFB_PAIR
+    return p;
+}
+
+inline termwise::Rates<F2> pairRates(const termwise::Rates<float>& r)
+{
+    termwise::Rates<F2> p;
+#define VFB_PAIR(name) p.name = F2(r.name);
+    VFB_K17_TERM_RATES(VFB_PAIR)
 #undef VFB_PAIR
     return p;
 }
