@@ -68,10 +68,15 @@ cudaError_t upload(T** dst, const std::vector<T>& v, cudaStream_t stream)
 
 // Tile configurations (tile width, stages, resident blocks) the library is
 // compiled for; 0 stages selects the direct-load kernel, 1 stage the paired
-// direct-load kernel.  Entry 12 (paired, four blocks per SM) is the default
-// for FP32, entry 19 (paired, five blocks) for the 16-bit storages and entry 1
-// for FP64 (the fastest at Taylor-Green 512^3 on B200: FP16 / FX16 33.5 G node
-// updates per second with entry 19 against 32.5 / 31.8 with entry 12);
+// direct-load kernel.  Entry 12 (paired; four blocks per SM, five for the
+// default K17 pass) is the default for FP32, entry 19 (paired, five blocks) for
+// the 16-bit storages (B200, Taylor-Green 192^3 / 256^3: FP16 33.9 G node
+// updates per second with entry 19, 33.6 with entry 12, 33.2 with entry 20;
+// BF16 35.8 / 34.5 / 33.0; FX16 25.8 / 25.1 / 25.1 with the velocity read out)
+// and entry 11 (direct loads, 128 registers, four blocks) for FP64 (224^3: 12.1
+// G with direct loads, 11.2 with the staged entry 1; 128^3: 11.7 and 11.4: since
+// a node's collision fits 128 registers, 16 resident warps hide the loads better
+// than one tile of look-ahead does for 8).
 // VFB_TILE_CONFIG=<index> selects another one at plan creation (used to tune
 // the shape on new hardware).
 struct TileConfigInfo {
@@ -82,7 +87,7 @@ static const TileConfigInfo kTileConfigs[] = {
     { 256, 2, 3, false }, { 128, 2, 2, true }, { 256, 3, 2, false }, { 192, 3, 3, false },
     { 160, 3, 4, false }, { 128, 4, 3, false }, { 128, 3, 3, true },
     // direct loads (0 stages)
-    { 128, 0, 4, false }, { 256, 0, 3, false }, { 128, 0, 6, false }, { 128, 0, 2, true }, { 128, 0, 3, true },
+    { 128, 0, 4, false }, { 256, 0, 3, false }, { 128, 0, 6, false }, { 128, 0, 2, true }, { 128, 0, 4, true },
     // paired direct loads (1 stage: T / 2 threads, two nodes each)
     { 256, 1, 4, false }, { 256, 1, 3, false }, { 256, 1, 2, false },
     // per-thread cp.async pipeline (2 shared-memory stages per thread)
@@ -97,7 +102,7 @@ static constexpr int kNumTileConfigs = (int)(sizeof(kTileConfigs) / sizeof(kTile
 static int chooseTileConfig(int storage)
 {
     const bool fp64 = storage == VFB_FP64;
-    int def = fp64 ? 1 : storage == VFB_FP32 ? 12 : 19;
+    int def = fp64 ? 11 : storage == VFB_FP32 ? 12 : 19;
     if (const char* env = std::getenv("VFB_TILE_CONFIG")) {
         const int c = std::atoi(env);
         if (c >= 0 && c < kNumTileConfigs && kTileConfigs[c].fp64 == fp64)
@@ -110,6 +115,8 @@ static int buildPlan(vfb_collision_plan_impl& p, int storage, const vfb_collisio
 {
     p.config = chooseTileConfig(storage);
     p.tileWidth = (uint32_t)kTileConfigs[p.config].T;
+    p.paired = kTileConfigs[p.config].stages == 1;
+    p.direct = kTileConfigs[p.config].stages == 0 || kTileConfigs[p.config].stages == 1;
     const unsigned long long N = a->numberOfLBnodes;
     const uint32_t nF = a->numberOfFluidNodes;
     std::vector<uint32_t> nx(N), ny(N), nz(N), fl(nF);
@@ -302,8 +309,8 @@ static int runPlanned(Op op, const vfb_collision_plan* plan, const vfb_collision
             return setError(VFB_ERR_INVALID_ARGUMENT, "template %d needs bodyForceX/Y/Z", t);
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (p.nLane) {
-        // the irregular nodes, one per thread through the index chain
+    if (p.nLane && !lanesInTileLaunch(p)) {
+        // the irregular nodes, one per thread by the generic kernel
         vfb_collision_args lane = *c;
         lane.fluidNodeIndices = p.laneList;
         lane.numberOfFluidNodes = p.nLane;
@@ -391,10 +398,11 @@ cudaError_t download(std::vector<T>& v, const void* src, size_t n, cudaStream_t 
 }
 
 // the tile configurations whose kernels run the BC epilogue: the paired
-// kernels (one stage) and the staged kernels (entries 0-6)
+// kernels (one stage) and the staged kernels (entries 0-6, and entry 11, whose
+// plan then runs the staged kernel)
 bool epilogueConfig(int c)
 {
-    return (c >= 0 && c <= 6) || c == 12 || c == 13 || c == 14 || c == 19 || c == 20;
+    return (c >= 0 && c <= 6) || c == 11 || c == 12 || c == 13 || c == 14 || c == 19 || c == 20;
 }
 } // namespace
 

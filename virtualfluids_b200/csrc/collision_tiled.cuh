@@ -21,13 +21,14 @@
 // lane list, collided one node per thread through the index chain by the
 // generic kernel.
 //
-// Two kernels consume the plan.  In the staged kernel (the FP32 / FP64
-// default) each block owns shared-memory stages with an mbarrier pair each;
-// blocks of a persistent grid stride over the tiles.  In the direct kernel
-// (the FP16 / BF16 default, where the collision arithmetic and not the memory
-// bounds the step) each block takes one tile and its warps load their values
-// from global memory straight into registers.  The arithmetic is the same
-// k17Collide / bgkCollide as the generic kernel.  Every population location
+// Three kernels consume the plan.  In the direct kernel (the FP64 default)
+// each block takes one tile and its warps load their values from global memory
+// straight into registers; the paired kernel (the default of the FP32
+// arithmetic) does the same with two nodes a thread.  In the staged kernel
+// (FP64 with the BC epilogue, tuning configurations) each block owns
+// shared-memory stages with an mbarrier pair each; blocks of a persistent grid
+// stride over the tiles.  The arithmetic is the same k17Collide / bgkCollide
+// as the generic kernel.  Every population location
 // is read and written by exactly one node, and a thread uses only the values
 // at its own node's locations, so values a bulk copy fetches for positions no
 // thread uses may be stale without harm.
@@ -141,6 +142,14 @@ struct TiledArgs {
     const BcEpilogue* epi;
     const uint32_t* epiTileStart;
     const uint32_t* epiTileNodes;
+    // the plan's lane list (irregular nodes) with its location table (8 x
+    // nLane), collided by the first laneBlocks blocks of the launch (the
+    // direct and paired kernels; 0: by a launch of its own)
+    const uint32_t* laneList;
+    const uint32_t* laneTable;
+    uint32_t nLane;
+    uint32_t laneBlocks;
+    bool offsets32; // a slot is at most 2^32 bytes long
 };
 
 // offset of location loc (bit 0 x, bit 1 y, bit 2 z) from the node for the
@@ -214,6 +223,27 @@ __device__ __forceinline__ void collideNode(const TiledArgs<S>& a, typename Stor
     } else {
         bgkCollide<R>(f, a.rates.omega);
     }
+}
+
+// entry i of the plan's lane list, through its location table
+template <class S, bool EVEN, Op OP, bool WM, bool BF>
+__device__ __forceinline__ void collideLane(const TiledArgs<S>& a, uint32_t i)
+{
+    if (i >= a.nLane)
+        return;
+    const uint32_t node = __ldg(a.laneList + i);
+    Locs L;
+#pragma unroll
+    for (int l = 0; l < 8; ++l)
+        L.k[l] = __ldg(a.laneTable + (unsigned long long)l * a.nLane + i);
+    typename Storage<S>::R f[27];
+#pragma unroll
+    for (int d = 0; d < 27; ++d)
+        f[d] = Storage<S>::load(a.sbase[d] + L.k[loc(d)], d);
+    collideNode<S, EVEN, OP, WM, BF>(a, f, node);
+#pragma unroll
+    for (int d = 0; d < 27; ++d)
+        Storage<S>::store(a.sbase[d] + L.k[loc(d)], f[inv(d)], d);
 }
 
 // Pipeline of one block: thread 0 is the producer.  Before refilling a stage
@@ -344,7 +374,8 @@ __global__ void __launch_bounds__(C::T, C::MINB) tiledKernel(const TiledArgs<S> 
 // block per tile, every warp loads its nodes' 27 values straight from global
 // memory into registers (coalesced: consecutive lanes read consecutive
 // addresses of each direction's run), collides and stores.  No producer, no
-// shared memory; latency is hidden by the warps resident on the SM.
+// shared memory; latency is hidden by the warps resident on the SM.  The first
+// laneBlocks blocks collide the plan's lane list through its location table.
 template <class S, class C, bool EVEN, Op OP, bool WM, bool BF>
 __global__ void __launch_bounds__(C::T, C::MINB) directKernel(const TiledArgs<S> a)
 {
@@ -352,8 +383,12 @@ __global__ void __launch_bounds__(C::T, C::MINB) directKernel(const TiledArgs<S>
     using R = typename Storage<S>::R;
     constexpr int WARPS = C::T / 32;
     const int tid = threadIdx.x;
+    if (blockIdx.x < a.laneBlocks) {
+        collideLane<S, EVEN, OP, WM, BF>(a, blockIdx.x * C::T + tid);
+        return;
+    }
     const int warp = tid >> 5, lane = tid & 31;
-    const uint32_t* meta = a.meta + (size_t)blockIdx.x * C::META_WORDS;
+    const uint32_t* meta = a.meta + (size_t)(blockIdx.x - a.laneBlocks) * C::META_WORDS;
     const bool active = (__ldg(meta + 4 + warp) >> lane) & 1u;
     if (!active)
         return;
@@ -393,6 +428,13 @@ __global__ void __launch_bounds__(C::T, C::MINB) directKernel(const TiledArgs<S>
 // loads and stores without predicates, the second node's address an
 // immediate offset from the first's.  Other warps take the general path:
 // per-lane predicates and the lanes' location offsets.
+//
+// The first laneBlocks blocks collide the plan's lane list, one entry a thread
+// in scalar arithmetic: as part of this launch its latency lies under the
+// tiles' instead of in a launch before them (a 24^3 cavity's two steps took
+// 23.9 us with that launch and 18.4 us without).  They come first so that they
+// do not form the launch's tail, and share no code with the tiles' path, whose
+// registers (96 at five blocks) a common path raised by 11.
 template <class S, class C, bool EVEN, Op OP, bool WM, bool BF, bool EPI = false>
 __global__ void __launch_bounds__(C::T / 2, C::MINB) pairKernel(const TiledArgs<S> a)
 {
@@ -402,7 +444,12 @@ __global__ void __launch_bounds__(C::T / 2, C::MINB) pairKernel(const TiledArgs<
     constexpr int WARPS = C::T / 32;
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    const uint32_t* meta = a.meta + (size_t)blockIdx.x * C::META_WORDS;
+    if (blockIdx.x < a.laneBlocks) {
+        collideLane<S, EVEN, OP, WM, BF>(a, blockIdx.x * HALF + tid);
+        return;
+    }
+    const uint32_t tile = blockIdx.x - a.laneBlocks;
+    const uint32_t* meta = a.meta + (size_t)tile * C::META_WORDS;
     const uint32_t maskA = __ldg(meta + 4 + warp), maskB = __ldg(meta + 4 + W2 + warp);
     const bool actA = (maskA >> lane) & 1u;
     const bool actB = (maskB >> lane) & 1u;
@@ -415,7 +462,7 @@ __global__ void __launch_bounds__(C::T / 2, C::MINB) pairKernel(const TiledArgs<
     const uint32_t wf = __ldg(meta + 1);
     const bool wrap = (((wf >> warp) | (wf >> (W2 + warp))) & 1u) != 0;
     // the same for every lane of the warp
-    const bool full = !wrap && (maskA & maskB) == 0xffffffffu;
+    const bool full = !wrap && (maskA & maskB) == 0xffffffffu && a.offsets32;
     LaneOffsets oA = laneOffsets(a, 0), oB = oA;
     if (wrap) {
         auto bitsOf = [&](int word) {
@@ -426,13 +473,18 @@ __global__ void __launch_bounds__(C::T / 2, C::MINB) pairKernel(const TiledArgs<
         oA = laneOffsets(a, bitsOf(warp));
         oB = laneOffsets(a, bitsOf(W2 + warp));
     }
+    // a full warp's location of direction d of node A: a launch constant plus a
+    // 32-bit byte offset (an address register less per access than with a
+    // 64-bit index; slots beyond 2^32 bytes take the general path)
+    const uint32_t byteOffset = kA * (uint32_t)sizeof(S);
+    auto at = [&](int d) { return reinterpret_cast<S*>(reinterpret_cast<char*>(a.gbase[d]) + byteOffset); };
     // a 16-bit format's storage scale is applied to both nodes in one paired multiply
     using St = Storage<S>;
     F2 f[27];
     if (full) {
 #pragma unroll
         for (int d = 0; d < 27; ++d) {
-            const S* p = a.gbase[d] + kA;
+            const S* p = at(d);
             f[d] = F2(St::loadRaw(p), St::loadRaw(p + HALF));
         }
     } else {
@@ -488,7 +540,7 @@ __global__ void __launch_bounds__(C::T / 2, C::MINB) pairKernel(const TiledArgs<
     if (full) {
 #pragma unroll
         for (int d = 0; d < 27; ++d) {
-            S* p = a.gbase[d] + kA;
+            S* p = at(d);
             const F2 v = f[inv(d)];
             St::storeRaw(p, v.v.x);
             St::storeRaw(p + HALF, v.v.y);
@@ -509,7 +561,7 @@ __global__ void __launch_bounds__(C::T / 2, C::MINB) pairKernel(const TiledArgs<
     // global stores visible to all its threads).  The values are re-read from
     // L1 / L2, and no lane waits on another lane's BC node of the same warp.
     if constexpr (EPI) {
-        const uint32_t b = __ldg(a.epiTileStart + blockIdx.x), e = __ldg(a.epiTileStart + blockIdx.x + 1);
+        const uint32_t b = __ldg(a.epiTileStart + tile), e = __ldg(a.epiTileStart + tile + 1);
         if (b != e) {
             __syncthreads();
             for (uint32_t j = b + tid; j < e; j += HALF)
@@ -605,6 +657,8 @@ __global__ void __launch_bounds__(C::T, C::MINB) asyncKernel(const TiledArgs<S> 
 struct vfb_collision_plan_impl {
     int storage = 0;
     int config = 0;      // index into kTileConfigs
+    bool direct = false; // the configuration's kernel is the direct or the paired one
+    bool paired = false; // the paired one
     uint32_t tileWidth = 256;
     uint32_t metaWords = 12;
     unsigned long long N = 0;
@@ -634,6 +688,15 @@ struct vfb_collision_plan_impl {
     unsigned long long epiCount[2] = { 0, 0 }; // nodes, records
 };
 
+// whether the plan's tile kernel collides the lane list too (the direct and
+// the paired kernels; the persistent ones leave it to the generic kernel)
+inline bool lanesInTileLaunch(const vfb_collision_plan_impl& p)
+{
+    if (p.storage == VFB_FP64)
+        return p.direct && !p.epi;
+    return p.direct;
+}
+
 template <class S, class C, bool EVEN, Op OP, bool WM, bool BF, bool EPI = false>
 static int launchTiledT(const TiledArgs<S>& a, cudaStream_t stream)
 {
@@ -655,14 +718,14 @@ static int launchTiledT(const TiledArgs<S>& a, cudaStream_t stream)
         launchDependent(asyncKernel<S, C, EVEN, OP, WM, BF>, std::max(1u, grid), C::T, smem, stream, a);
         return checkLaunch("pipelined planned collision");
     } else if constexpr (C::STAGES == 1 && sizeof(S) <= 4) {
-        launchDependent(pairKernel<S, C, EVEN, OP, WM, BF, EPI>, a.nTiles, C::T / 2, 0, stream, a);
+        launchDependent(pairKernel<S, C, EVEN, OP, WM, BF, EPI>, a.laneBlocks + a.nTiles, C::T / 2, 0, stream, a);
         return checkLaunch("paired planned collision");
     } else if constexpr (C::STAGES == 1) {
         // the paired form computes in FP32: FP64 storage uses the staged kernel
         // of the same tile width (same metadata layout and copy geometry)
         return launchTiledT<S, TileCfg<S, C::T, 2, 3>, EVEN, OP, WM, BF, EPI>(a, stream);
     } else if constexpr (C::STAGES == 0) {
-        launchDependent(directKernel<S, C, EVEN, OP, WM, BF>, a.nTiles, C::T, 0, stream, a);
+        launchDependent(directKernel<S, C, EVEN, OP, WM, BF>, a.laneBlocks + a.nTiles, C::T, 0, stream, a);
         return checkLaunch("direct planned collision");
     } else {
     static int blocks = 0;
@@ -812,18 +875,28 @@ static int launchTiled(Op op, const vfb_collision_plan_impl& p, const vfb_collis
     a.epi = p.epi;
     a.epiTileStart = p.epiTileStart;
     a.epiTileNodes = p.epiTileNodes;
-    if (p.nTiles == 0)
+    a.offsets32 = p.N * sizeof(S) <= 0xffffffffull;
+    a.laneList = p.laneList;
+    a.laneTable = p.laneLocations;
+    a.nLane = p.nLane;
+    // lane entries per block: its threads (the paired kernel's blocks have T / 2)
+    const uint32_t perBlock = sizeof(S) == 8 || !p.paired ? p.tileWidth : p.tileWidth / 2;
+    a.laneBlocks = lanesInTileLaunch(p) ? (p.nLane + perBlock - 1) / perBlock : 0;
+    if (p.nTiles + a.laneBlocks == 0)
         return VFB_OK;
     const bool even = c->isEvenTimestep != 0;
     const int t = c->collisionTemplate;
     if constexpr (sizeof(S) == 8) {
+        // the BC epilogue exists for the staged kernel (the same tiles)
+        if (p.epi)
+            return dispatchTuning<S, TileCfg<S, 128, 2, 2>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         switch (p.config) {
+        case 1: return dispatchTiled<S, TileCfg<S, 128, 2, 2>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 6: return dispatchTuning<S, TileCfg<S, 128, 3, 3>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 10: return dispatchTuning<S, TileCfg<S, 128, 0, 2>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
-        case 11: return dispatchTuning<S, TileCfg<S, 128, 0, 3>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 17: return dispatchTuning<S, TileCfg<S, 128, 2, 3, 1>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 18: return dispatchTuning<S, TileCfg<S, 128, 2, 2, 1>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
-        default: return dispatchTiled<S, TileCfg<S, 128, 2, 2>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
+        default: return dispatchTiled<S, TileCfg<S, 128, 0, 4>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         }
     } else {
         switch (p.config) {
@@ -832,7 +905,12 @@ static int launchTiled(Op op, const vfb_collision_plan_impl& p, const vfb_collis
         case 4: return dispatchTuning<S, TileCfg<S, 160, 3, 4>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 5: return dispatchTuning<S, TileCfg<S, 128, 4, 3>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 7: return dispatchTuning<S, TileCfg<S, 128, 0, 4>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
-        case 12: return dispatchTiled<S, TileCfg<S, 256, 1, 4>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
+        case 12:
+            // FP32: the K17 pass at five blocks per SM (B200, 256^3: 26.0 G node
+            // updates/s against 25.4 at four), BGK at four (25.8 against 24.0)
+            if (sizeof(S) == 4 && op == Op::K17 && t == VFB_TEMPLATE_DEFAULT)
+                return dispatchTiled<S, TileCfg<S, 256, 1, 5>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
+            return dispatchTiled<S, TileCfg<S, 256, 1, 4>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 15:
             if constexpr (sizeof(S) == 4)
                 return dispatchTuning<S, TileCfg<S, 256, 2, 3, 1>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
