@@ -101,15 +101,20 @@ __host__ __device__ __forceinline__ void cornerSums(const R* q, R* out)
 // index of a sum in cornerSums' output
 enum CornerSum : int { S1 = 0, SX = 1, SY = 2, SXY = 3, SZ = 4, SXZ = 5, SYZ = 6, SXYZ = 7 };
 
-// MomentsOnSourceNodeSet::calculateCoefficients (InterpolationCoefficients.h:201-430)
+// the signed corner sums of the nine quantities (indexed by CornerSum)
 template <class R>
-__host__ __device__ __forceinline__ InterpCoeffs<R> interpolationCoefficients(const SourceMoments<R>* src, R xoff,
-                                                                              R yoff, R zoff)
+struct SourceSums {
+    R vx[8], vy[8], vz[8], dr[8], kxy[8], kyz[8], kxz[8], kmy[8], kmz[8];
+};
+
+template <class R>
+__host__ __device__ __forceinline__ SourceSums<R> sourceSums(const SourceMoments<R>* src)
 {
-    R q[8], vx[8], vy[8], vz[8], dr[8], kxy[8], kyz[8], kxz[8], kmy[8], kmz[8];
+    SourceSums<R> s;
+    R q[8];
 #define VFB_CORNERS(OUT, FIELD)                                                                                        \
     _Pragma("unroll") for (int c = 0; c < 8; ++c) q[c] = src[c].FIELD;                                                 \
-    cornerSums(q, OUT);
+    cornerSums(q, s.OUT);
     VFB_CORNERS(vx, vx)
     VFB_CORNERS(vy, vy)
     VFB_CORNERS(vz, vz)
@@ -120,6 +125,18 @@ __host__ __device__ __forceinline__ InterpCoeffs<R> interpolationCoefficients(co
     VFB_CORNERS(kmy, kxxMyy)
     VFB_CORNERS(kmz, kxxMzz)
 #undef VFB_CORNERS
+    return s;
+}
+
+// MomentsOnSourceNodeSet::calculateCoefficients (InterpolationCoefficients.h:201-430).
+// Reads every sum of the velocities and the density and, of the second moments,
+// kxy[SX, SY], kyz[SY, SZ], kxz[SX, SZ], kmy and kmz[SX, SY, SZ].
+template <class R>
+__host__ __device__ __forceinline__ InterpCoeffs<R> interpolationCoefficients(const SourceSums<R>& sums, R xoff, R yoff,
+                                                                              R zoff)
+{
+    const R *vx = sums.vx, *vy = sums.vy, *vz = sums.vz, *dr = sums.dr, *kxy = sums.kxy, *kyz = sums.kyz,
+            *kxz = sums.kxz, *kmy = sums.kmy, *kmz = sums.kmz;
     InterpCoeffs<R> k;
     k.a000 = (R(2) * (((vy[SXY] + vz[SXZ]) - kxy[SY]) - kxz[SZ]) + R(8) * vx[S1] - (kmy[SX] + kmz[SX])) / R(64);
     k.b000 = (R(2) * (((kmy[SY] + vx[SXY]) + vz[SYZ]) - (kxy[SX] + kyz[SZ])) + R(8) * vy[S1] - kmz[SY]) / R(64);

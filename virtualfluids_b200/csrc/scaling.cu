@@ -145,7 +145,7 @@ __host__ __device__ __forceinline__ void coarseToFineCell(const ScalingView<S, R
     blockWalk(v.coarseCells[i], v.nXc, v.nYc, v.nZc, B);
     SourceMoments<R> src[8];
     cellSourceMoments<A, EVEN_C>(v.distC, v.NC, B, v.omegaC, src);
-    const InterpCoeffs<R> k = interpolationCoefficients(src, v.offX[i], v.offY[i], v.offZ[i]);
+    const InterpCoeffs<R> k = interpolationCoefficients(sourceSums(src), v.offX[i], v.offY[i], v.offZ[i]);
     blockWalk(v.fineCells[i], v.nXf, v.nYf, v.nZf, B);
     const uint8_t* writes = v.mask ? v.mask + 27 * (size_t)i : nullptr;
 #pragma unroll
@@ -170,7 +170,7 @@ __host__ __device__ __forceinline__ void fineToCoarseCell(const ScalingView<S, R
     blockWalk(v.fineCells[i], v.nXf, v.nYf, v.nZf, B);
     SourceMoments<R> src[8];
     cellSourceMoments<A, true>(v.distF, v.NF, B, v.omegaF, src);
-    const InterpCoeffs<R> k = interpolationCoefficients(src, v.offX[i], v.offY[i], v.offZ[i]);
+    const InterpCoeffs<R> k = interpolationCoefficients(sourceSums(src), v.offX[i], v.offY[i], v.offZ[i]);
     R f[27];
     interpolateFineToCoarse(f, k, v.omegaC);
     // the coarse node's own eight locations
@@ -192,31 +192,61 @@ __host__ __device__ __forceinline__ void fineToCoarseCell(const ScalingView<S, R
 // The device kernels give each cell eight threads (lanes 8g .. 8g + 7 of a
 // warp, corner c = lane % 8): each thread walks the cell's block, loads the
 // 27 populations of its own source corner and forms that corner's moments;
-// the group gathers the eight moment sets with shuffles, every thread forms
-// the same coefficients (interpolationCoefficients on the same eight sets, so
+// the group forms the signed corner sums by shuffles, every thread forms
+// the same coefficients (interpolationCoefficients on the same sums, so
 // the same values as the one-thread cell functions above), and the writes
 // are shared out: fine corner c (coarse to fine) or the coarse node's
 // directions d with d % 8 == c (fine to coarse).  Eight times the threads of
 // a cell per cell keep eight times the loads in flight.
 constexpr int kScalingThreads = 128; // 16 cells per block
 
-// the eight corners' moments of the group of this lane, from each lane's own
+// The signed corner sums of one quantity over the group of this lane: a
+// butterfly across the eight lanes (the additions of cornerSums in its order),
+// after which lane m holds the sum of index m
 template <class R>
-__device__ __forceinline__ void gatherMoments(const SourceMoments<R>& mine, SourceMoments<R>* src)
+__device__ __forceinline__ R laneCornerSum(R q)
+{
+#pragma unroll
+    for (int bit = 1; bit < 8; bit <<= 1) {
+        const R other = __shfl_xor_sync(0xffffffffu, q, bit);
+        q = fma((threadIdx.x & bit) ? R(-1) : R(1), other, q);
+    }
+    return q;
+}
+
+// all sums the coefficients read, in every lane: each quantity's butterfly,
+// then the sums from the lanes that hold them (27 additions a lane instead of
+// the 216 of forming every sum in every lane from the corners' values)
+template <class R>
+__device__ __forceinline__ SourceSums<R> gatherSums(const SourceMoments<R>& mine)
 {
     const int base = (int)(threadIdx.x & 31u) & ~7;
+    SourceSums<R> s;
+    auto from = [&](R v, int m) { return __shfl_sync(0xffffffffu, v, base + m); };
+    const R vx = laneCornerSum(mine.vx), vy = laneCornerSum(mine.vy), vz = laneCornerSum(mine.vz);
+    const R dr = laneCornerSum(mine.drho);
+    const R kxy = laneCornerSum(mine.kxy), kyz = laneCornerSum(mine.kyz), kxz = laneCornerSum(mine.kxz);
+    const R kmy = laneCornerSum(mine.kxxMyy), kmz = laneCornerSum(mine.kxxMzz);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        src[c].drho = __shfl_sync(0xffffffffu, mine.drho, base + c);
-        src[c].vx = __shfl_sync(0xffffffffu, mine.vx, base + c);
-        src[c].vy = __shfl_sync(0xffffffffu, mine.vy, base + c);
-        src[c].vz = __shfl_sync(0xffffffffu, mine.vz, base + c);
-        src[c].kxy = __shfl_sync(0xffffffffu, mine.kxy, base + c);
-        src[c].kyz = __shfl_sync(0xffffffffu, mine.kyz, base + c);
-        src[c].kxz = __shfl_sync(0xffffffffu, mine.kxz, base + c);
-        src[c].kxxMyy = __shfl_sync(0xffffffffu, mine.kxxMyy, base + c);
-        src[c].kxxMzz = __shfl_sync(0xffffffffu, mine.kxxMzz, base + c);
+    for (int m = 0; m < 8; ++m) {
+        s.vx[m] = from(vx, m);
+        s.vy[m] = from(vy, m);
+        s.vz[m] = from(vz, m);
+        s.dr[m] = from(dr, m);
     }
+    s.kxy[SX] = from(kxy, SX);
+    s.kxy[SY] = from(kxy, SY);
+    s.kyz[SY] = from(kyz, SY);
+    s.kyz[SZ] = from(kyz, SZ);
+    s.kxz[SX] = from(kxz, SX);
+    s.kxz[SZ] = from(kxz, SZ);
+    s.kmy[SX] = from(kmy, SX);
+    s.kmy[SY] = from(kmy, SY);
+    s.kmy[SZ] = from(kmy, SZ);
+    s.kmz[SX] = from(kmz, SX);
+    s.kmz[SY] = from(kmz, SY);
+    s.kmz[SZ] = from(kmz, SZ);
+    return s;
 }
 
 // the eight locations of corner c of a block (a switch over the lane's corner
@@ -286,22 +316,31 @@ __device__ __forceinline__ void coarseToFineBlock(const ScalingView<S, typename 
     const uint32_t ic = active ? i : v.nCells - 1;
     uint32_t Lc[8];
     cellCornerLocations(v.blocksC, v.coarseCells, v.nXc, v.nYc, v.nZc, ic, c, Lc);
-    SourceMoments<R> src[8];
-    gatherMoments(cornerMoments<EVEN_C>(v.distC, v.NC, Lc, v.omegaC), src);
-    const InterpCoeffs<R> k = interpolationCoefficients(src, v.offX[ic], v.offY[ic], v.offZ[ic]);
+    // where the results go, loaded beside the sources rather than after the arithmetic
+    uint32_t Lf[8];
+    cellCornerLocations(v.blocksF, v.fineCells, v.nXf, v.nYf, v.nZf, ic, c, Lf);
+    uint32_t writes = 0x7ffffffu;
+    if (v.mask) {
+        const uint8_t* row = v.mask + 27 * (size_t)ic;
+        writes = 0;
+#pragma unroll
+        for (int d = 0; d < 27; ++d)
+            writes |= (uint32_t)((__ldg(row + d) >> c) & 1) << d;
+    }
+    const R xoff = v.offX[ic], yoff = v.offY[ic], zoff = v.offZ[ic];
+    const SourceSums<R> sums = gatherSums(cornerMoments<EVEN_C>(v.distC, v.NC, Lc, v.omegaC));
     if (!active)
         return;
-    cellCornerLocations(v.blocksF, v.fineCells, v.nXf, v.nYf, v.nZf, ic, c, Lc);
+    const InterpCoeffs<R> k = interpolationCoefficients(sums, xoff, yoff, zoff);
     const R x = (c & 1) ? R(1) / R(4) : -R(1) / R(4);
     const R y = (c & 2) ? R(1) / R(4) : -R(1) / R(4);
     const R z = (c & 4) ? R(1) / R(4) : -R(1) / R(4);
     R f[27];
     interpolateCoarseToFine(f, k, v.omegaF, x, y, z);
-    const uint8_t* writes = v.mask ? v.mask + 27 * (size_t)ic : nullptr;
 #pragma unroll
     for (int d = 0; d < 27; ++d)
-        if (!writes || ((writes[d] >> c) & 1))
-            Storage<S>::store(v.distF + (unsigned long long)slot<true>(d) * v.NF + Lc[loc(d)], f[d], d);
+        if ((writes >> d) & 1)
+            Storage<S>::store(v.distF + (unsigned long long)slot<true>(d) * v.NF + Lf[loc(d)], f[d], d);
 }
 
 template <class S, bool EVEN_C>
@@ -314,16 +353,16 @@ __device__ __forceinline__ void fineToCoarseBlock(const ScalingView<S, typename 
     const uint32_t ic = active ? i : v.nCells - 1;
     uint32_t Lc[8];
     cellCornerLocations(v.blocksF, v.fineCells, v.nXf, v.nYf, v.nZf, ic, c, Lc);
-    SourceMoments<R> src[8];
-    gatherMoments(cornerMoments<true>(v.distF, v.NF, Lc, v.omegaF), src);
-    const InterpCoeffs<R> k = interpolationCoefficients(src, v.offX[ic], v.offY[ic], v.offZ[ic]);
-    if (!active)
-        return;
-    R f[27];
-    interpolateFineToCoarse(f, k, v.omegaC);
     // the coarse node's own eight locations (corner 0 of its block)
     uint32_t L[8];
     cellCornerLocations(v.blocksC, v.coarseCells, v.nXc, v.nYc, v.nZc, ic, 0, L);
+    const R xoff = v.offX[ic], yoff = v.offY[ic], zoff = v.offZ[ic];
+    const SourceSums<R> sums = gatherSums(cornerMoments<true>(v.distF, v.NF, Lc, v.omegaF));
+    if (!active)
+        return;
+    const InterpCoeffs<R> k = interpolationCoefficients(sums, xoff, yoff, zoff);
+    R f[27];
+    interpolateFineToCoarse(f, k, v.omegaC);
 #pragma unroll
     for (int d = 0; d < 27; ++d)
         if ((d & 7) == c)
