@@ -32,7 +32,9 @@
 #include "adjoint_ops.gen.cuh"
 #include "capi_common.cuh"
 #include "d3q27.cuh"
+#include "pair32.cuh"
 #include "pdl.cuh"
+#include "tma.cuh"
 
 namespace vfb
 {
@@ -133,6 +135,63 @@ __global__ void __launch_bounds__(kThreads)
         dist[cell<R>(slot<EVEN>(d), N, L.k[loc(d)])] = f[inv(d)];
 }
 
+// The same for FP32 in paired arithmetic: thread t of a block takes the entries
+// t and t + kThreads of its 2 kThreads, whose values, tape and results it
+// handles together (k17Collide on a register pair issues about half the
+// instructions of two scalar ones, which bounded the scalar form: 31 us for the
+// channel's 522,560 nodes with or without the tape's 56 MB).
+template <bool EVEN>
+__global__ void __launch_bounds__(kThreads, 4)
+    tapeCollisionPairKernel(float* __restrict__ dist, unsigned long long N, const uint32_t* __restrict__ table,
+                            uint32_t n, const K17Rates<F2> r, float fx, float fy, float fz, float* __restrict__ tape)
+{
+    gridDependencyWait();
+    const uint32_t i = blockIdx.x * (2 * kThreads) + threadIdx.x;
+    if (i >= n)
+        return;
+    const bool both = i + kThreads < n;
+    const uint32_t j = both ? i + kThreads : i;
+    F2 f[27];
+    {
+        Locs A, B;
+#pragma unroll
+        for (int l = 0; l < 8; ++l) {
+            A.k[l] = __ldg(table + (unsigned long long)l * n + i);
+            B.k[l] = __ldg(table + (unsigned long long)l * n + j);
+        }
+#pragma unroll
+        for (int d = 0; d < 27; ++d) {
+            const float* p = dist + (unsigned long long)slot<EVEN>(d) * N;
+            f[d] = F2(p[A.k[loc(d)]], p[B.k[loc(d)]]);
+        }
+    }
+    if (tape) {
+#pragma unroll
+        for (int d = 0; d < 27; ++d) {
+            float* p = tape + (unsigned long long)d * n;
+            p[i] = f[d].v.x;
+            if (both)
+                p[j] = f[d].v.y;
+        }
+    }
+    F2 drho, ux, uy, uz;
+    k17Collide<F2>(f, r, F2(fx), F2(fy), F2(fz), drho, ux, uy, uz);
+    // the locations again, rather than 16 registers held over the collision
+    Locs A, B;
+#pragma unroll
+    for (int l = 0; l < 8; ++l) {
+        A.k[l] = tma::ldgOrdered(table + (unsigned long long)l * n + i);
+        B.k[l] = tma::ldgOrdered(table + (unsigned long long)l * n + j);
+    }
+#pragma unroll
+    for (int d = 0; d < 27; ++d) {
+        float* p = dist + (unsigned long long)slot<EVEN>(d) * N;
+        p[A.k[loc(d)]] = f[inv(d)].v.x;
+        if (both)
+            p[B.k[loc(d)]] = f[inv(d)].v.y;
+    }
+}
+
 // MINB: resident blocks per SM the register allocation aims at (the reverse
 // sweep wants more than 128 registers a thread; fewer registers spill to
 // local memory but hide more latency)
@@ -165,14 +224,19 @@ __global__ void __launch_bounds__(kThreads, MINB)
         gy = (double)gfy;
         gz = (double)gfz;
     }
-    gx = blockSum(gx);
-    gy = blockSum(gy);
-    gz = blockSum(gz);
-    // accumulated over the steps of a backward pass, each block in step order
-    if (threadIdx.x == 0) {
-        partials[3 * blockIdx.x + 0] += gx;
-        partials[3 * blockIdx.x + 1] += gy;
-        partials[3 * blockIdx.x + 2] += gz;
+    // accumulated over the steps of a backward pass, each warp in step order
+    // (a sum per warp: a block's would wait at two barriers a component)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        gx += __shfl_down_sync(0xffffffffu, gx, o);
+        gy += __shfl_down_sync(0xffffffffu, gy, o);
+        gz += __shfl_down_sync(0xffffffffu, gz, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        double* p = partials + 3ull * (i / 32);
+        p[0] += gx;
+        p[1] += gy;
+        p[2] += gz;
     }
 }
 
@@ -275,8 +339,11 @@ __global__ void __launch_bounds__(kThreads)
         postGatherEntry<R, EVEN>(lam, lat, bcK, table, q, n, tmp, i);
 }
 
-template <class R, int KIND, bool EVEN>
-__device__ __forceinline__ void postScatterEntry(R* __restrict__ lam, const BcLattice<R>& lat,
+// FUSED: the gather as well (tmp unused): the entry takes lam at its written
+// cells itself and clears them.  Valid when no entry writes a cell an entry
+// reads (sim_adjoint.cu checks this); one launch and the pass through tmp less.
+template <class R, int KIND, bool EVEN, bool FUSED>
+__device__ __forceinline__ void postScatterEntry(R* lam, const BcLattice<R>& lat,
                                                  const int32_t* __restrict__ bcK, const uint32_t* __restrict__ table,
                                                  const R* __restrict__ q, uint32_t n, const R* __restrict__ rec,
                                                  const R* __restrict__ tmp, double* __restrict__ gV, uint32_t i)
@@ -288,6 +355,27 @@ __device__ __forceinline__ void postScatterEntry(R* __restrict__ lam, const BcLa
         g[d] = rec[(unsigned long long)d * n + i];
         gg[d] = R(0);
     }
+    // all q values first: loads issued together, not one per loop iteration
+    R qv[26], tv[26];
+#pragma unroll
+    for (int j = 0; j < 26; ++j)
+        qv[j] = __ldg(q + (unsigned long long)qOrder(j) * n + i);
+    // the adjoints of the written cells, likewise; cleared after all of them are
+    // read (a store between two loads would hold the later load back)
+#pragma unroll
+    for (int j = 0; j < 26; ++j) {
+        const int d = qOrder(j);
+        tv[j] = R(0);
+        if (!(qv[j] >= R(0) && qv[j] <= R(1)))
+            continue;
+        tv[j] = FUSED ? lam[cell<R>(slot<!EVEN>(inv(d)), lat.N, L.k[loc(inv(d))])] : tmp[(unsigned long long)d * n + i];
+    }
+    if (FUSED) {
+#pragma unroll
+        for (int j = 0; j < 26; ++j)
+            if (qv[j] >= R(0) && qv[j] <= R(1))
+                lam[cell<R>(slot<!EVEN>(inv(qOrder(j))), lat.N, L.k[loc(inv(qOrder(j)))])] = R(0);
+    }
     R drho, vx1, vx2, vx3;
     bcMacros(g, drho, vx1, vx2, vx3);
     const R rho = R(1) + drho;
@@ -296,11 +384,6 @@ __device__ __forceinline__ void postScatterEntry(R* __restrict__ lam, const BcLa
     const R c1 = R(1) / (R(1) - omega);
     R gdrho = R(0), gux = R(0), guy = R(0), guz = R(0), gcuSq = R(0);
     R gUx = R(0), gUy = R(0), gUz = R(0);
-    // all q values first: loads issued together, not one per loop iteration
-    R qv[26];
-#pragma unroll
-    for (int j = 0; j < 26; ++j)
-        qv[j] = __ldg(q + (unsigned long long)qOrder(j) * n + i);
 #pragma unroll
     for (int j = 0; j < 26; ++j) {
         const int d = qOrder(j);
@@ -308,7 +391,7 @@ __device__ __forceinline__ void postScatterEntry(R* __restrict__ lam, const BcLa
         if (!(qd >= R(0) && qd <= R(1)))
             continue;
         const int e = inv(d);
-        const R t = tmp[(unsigned long long)d * n + i];
+        const R t = tv[j];
         const R w = weight<R>(d);
         const R r = linkReciprocal(R(1) + qd);
         const R A = (R(1) - qd) * r;
@@ -351,16 +434,16 @@ __device__ __forceinline__ void postScatterEntry(R* __restrict__ lam, const BcLa
     }
 }
 
-template <class R, int KIND, bool EVEN>
+template <class R, int KIND, bool EVEN, bool FUSED>
 __global__ void __launch_bounds__(kThreads)
-    postScatterKernel(R* __restrict__ lam, const BcLattice<R> lat, const int32_t* __restrict__ bcK,
+    postScatterKernel(R* lam, const BcLattice<R> lat, const int32_t* __restrict__ bcK,
                       const uint32_t* __restrict__ table, const R* __restrict__ q, uint32_t n,
                       const R* __restrict__ rec, const R* __restrict__ tmp, double* __restrict__ gV)
 {
     gridDependencyWait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n)
-        postScatterEntry<R, KIND, EVEN>(lam, lat, bcK, table, q, n, rec, tmp, gV, i);
+        postScatterEntry<R, KIND, EVEN, FUSED>(lam, lat, bcK, table, q, n, rec, tmp, gV, i);
 }
 
 // ------------------------------------------ post-collision lists together --
@@ -408,8 +491,8 @@ __global__ void __launch_bounds__(kThreads) postGatherListsKernel(R* __restrict_
         postGatherEntry<R, EVEN>(lam, lat, L.k, L.table, L.q, L.n, L.tmp, i);
 }
 
-template <class R, bool EVEN>
-__global__ void __launch_bounds__(kThreads) postScatterListsKernel(R* __restrict__ lam, const BcLattice<R> lat,
+template <class R, bool EVEN, bool FUSED>
+__global__ void __launch_bounds__(kThreads) postScatterListsKernel(R* lam, const BcLattice<R> lat,
                                                                    const PostLists<R> P)
 {
     gridDependencyWait();
@@ -418,27 +501,38 @@ __global__ void __launch_bounds__(kThreads) postScatterListsKernel(R* __restrict
     if (i >= L.n)
         return;
     if (L.kind == VFB_BC_VELOCITY_INTERPOLATED)
-        postScatterEntry<R, VFB_BC_VELOCITY_INTERPOLATED, EVEN>(lam, lat, L.k, L.table, L.q, L.n, L.rec, L.tmp,
+        postScatterEntry<R, VFB_BC_VELOCITY_INTERPOLATED, EVEN, FUSED>(lam, lat, L.k, L.table, L.q, L.n, L.rec, L.tmp,
                                                                 L.gV, i);
     else
-        postScatterEntry<R, VFB_BC_NOSLIP_INTERPOLATED, EVEN>(lam, lat, L.k, L.table, L.q, L.n, L.rec, L.tmp,
+        postScatterEntry<R, VFB_BC_NOSLIP_INTERPOLATED, EVEN, FUSED>(lam, lat, L.k, L.table, L.q, L.n, L.rec, L.tmp,
                                                               nullptr, i);
 }
 
 // --------------------------------------------------------------- pressure --
+// `table`: the list's locations (16 n: the node's eight, then its
+// neighbour's), eight independent loads instead of a chain through the
+// neighbour arrays
+__device__ __forceinline__ Locs tableLocations(const uint32_t* __restrict__ table, uint32_t n, uint32_t i)
+{
+    Locs L;
+#pragma unroll
+    for (int l = 0; l < 8; ++l)
+        L.k[l] = __ldg(table + (unsigned long long)l * n + i);
+    return L;
+}
+
 template <class R, bool EVEN>
 __global__ void __launch_bounds__(kThreads)
-    pressureKernel(R* __restrict__ dist, const BcLattice<R> lat, const int32_t* __restrict__ bcK,
-                   const int32_t* __restrict__ bcKN, const R* __restrict__ rhoBC, uint32_t n, int axis, int sgn,
-                   R* __restrict__ rec)
+    pressureKernel(R* __restrict__ dist, const BcLattice<R> lat, const uint32_t* __restrict__ table,
+                   const R* __restrict__ rhoBC, uint32_t n, int axis, int sgn, R* __restrict__ rec)
 {
     gridDependencyWait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
     const unsigned long long N = lat.N;
-    const Locs L = listIndices((uint32_t)__ldg(bcK + i), lat.nX, lat.nY, lat.nZ);
-    const Locs LN = listIndices((uint32_t)__ldg(bcKN + i), lat.nX, lat.nY, lat.nZ);
+    const Locs L = tableLocations(table, n, i);
+    const Locs LN = tableLocations(table + 8ull * n, n, i);
     R f[27];
 #pragma unroll
     for (int d = 0; d < 27; ++d)
@@ -460,14 +554,14 @@ __global__ void __launch_bounds__(kThreads)
 
 template <class R, bool EVEN>
 __global__ void __launch_bounds__(kThreads)
-    pressureGatherKernel(R* __restrict__ lam, const BcLattice<R> lat, const int32_t* __restrict__ bcK, uint32_t n,
+    pressureGatherKernel(R* __restrict__ lam, const BcLattice<R> lat, const uint32_t* __restrict__ table, uint32_t n,
                          int axis, int sgn, R* __restrict__ tmp)
 {
     gridDependencyWait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    const Locs L = listIndices((uint32_t)__ldg(bcK + i), lat.nX, lat.nY, lat.nZ);
+    const Locs L = tableLocations(table, n, i);
 #pragma unroll
     for (int d = 0; d < 27; ++d) {
         const int c = axis == 0 ? cx(d) : axis == 1 ? cy(d) : cz(d);
@@ -479,9 +573,11 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
-template <class R, bool EVEN>
+// FUSED: the gather as well (tmp unused), when no entry's neighbour is itself
+// an entry's node (sim_adjoint.cu checks this)
+template <class R, bool EVEN, bool FUSED>
 __global__ void __launch_bounds__(kThreads)
-    pressureScatterKernel(R* __restrict__ lam, const BcLattice<R> lat, const int32_t* __restrict__ bcKN,
+    pressureScatterKernel(R* lam, const BcLattice<R> lat, const uint32_t* __restrict__ table,
                           const R* __restrict__ rhoBC, uint32_t n, int axis, int sgn, const R* __restrict__ rec,
                           const R* __restrict__ tmp)
 {
@@ -489,7 +585,24 @@ __global__ void __launch_bounds__(kThreads)
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    const Locs LN = listIndices((uint32_t)__ldg(bcKN + i), lat.nX, lat.nY, lat.nZ);
+    const Locs LN = tableLocations(table + 8ull * n, n, i);
+    auto written = [&](int d) { return (axis == 0 ? cx(d) : axis == 1 ? cy(d) : cz(d)) != sgn; };
+    R tv[27];
+    {
+        const Locs L = tableLocations(table, n, i);
+        // all loads before the clearing stores (see postScatterEntry)
+#pragma unroll
+        for (int d = 0; d < 27; ++d)
+            tv[d] = !written(d) ? R(0)
+                    : FUSED     ? lam[cell<R>(slot<EVEN>(d), lat.N, L.k[loc(d)])]
+                                : tmp[(unsigned long long)d * n + i];
+        if (FUSED) {
+#pragma unroll
+            for (int d = 0; d < 27; ++d)
+                if (written(d))
+                    lam[cell<R>(slot<EVEN>(d), lat.N, L.k[loc(d)])] = R(0);
+        }
+    }
     R f[27], gf[27];
 #pragma unroll
     for (int d = 0; d < 27; ++d) {
@@ -507,7 +620,7 @@ __global__ void __launch_bounds__(kThreads)
         const int c = axis == 0 ? cx(d) : axis == 1 ? cy(d) : cz(d);
         if (c == sgn)
             continue;
-        const R t = tmp[(unsigned long long)d * n + i];
+        const R t = tv[d];
         const R w = weight<R>(d);
         const R cu = cdot<R>(d, ux, uy, uz);
         gf[d] += t;
@@ -593,7 +706,7 @@ int axisOf(int direction, int& axis, int& sgn)
 }
 } // namespace
 
-unsigned collisionBlocks(uint32_t nFluid) { return blocksFor(nFluid); }
+unsigned collisionPartials(uint32_t nFluid) { return blocksFor(nFluid) * (kThreads / 32); }
 unsigned objectiveBlocks(uint32_t n) { return blocksFor(n); }
 
 template <class R>
@@ -603,6 +716,18 @@ int collision(R* dist, unsigned long long N, const uint32_t* nX, const uint32_t*
 {
     if (nFluid == 0)
         return VFB_OK;
+    if constexpr (sizeof(R) == 4) {
+        if (loc) {
+            const unsigned b = (nFluid + 2 * kThreads - 1) / (2 * kThreads);
+            if (even)
+                launchDependent(tapeCollisionPairKernel<true>, b, kThreads, 0, s, dist, N, loc, nFluid,
+                                pairRates(rates), fx, fy, fz, tape);
+            else
+                launchDependent(tapeCollisionPairKernel<false>, b, kThreads, 0, s, dist, N, loc, nFluid,
+                                pairRates(rates), fx, fy, fz, tape);
+            return checkLaunch("adjoint forward collision");
+        }
+    }
     const unsigned b = blocksFor(nFluid);
     if (even)
         launchDependent(tapeCollisionKernel<R, true>, b, kThreads, 0, s, dist, N, nX, nY, nZ, fluid, loc, nFluid,
@@ -689,7 +814,12 @@ template <class R, int KIND, bool EVEN>
 void launchPostScatter(unsigned b, cudaStream_t s, R* lam, const BcLattice<R>& lat, const int32_t* k,
                        const uint32_t* table, const R* q, uint32_t n, const R* rec, const R* tmp, double* gV)
 {
-    launchDependent(postScatterKernel<R, KIND, EVEN>, b, kThreads, 0, s, lam, lat, k, table, q, n, rec, tmp, gV);
+    if (tmp)
+        launchDependent(postScatterKernel<R, KIND, EVEN, false>, b, kThreads, 0, s, lam, lat, k, table, q, n, rec,
+                        tmp, gV);
+    else
+        launchDependent(postScatterKernel<R, KIND, EVEN, true>, b, kThreads, 0, s, lam, lat, k, table, q, n, rec, tmp,
+                        gV);
 }
 
 template <class R>
@@ -705,12 +835,14 @@ int postBCAdjoint(int kind, R* lam, const BcLattice<R>& lat, const int32_t* k, c
     if (kind != VFB_BC_VELOCITY_INTERPOLATED && kind != VFB_BC_NOSLIP_INTERPOLATED)
         return setError(VFB_ERR_INVALID_ARGUMENT, "BC kind %d has no adjoint", kind);
     const unsigned b = blocksFor(n);
-    if (even)
-        launchDependent(postGatherKernel<R, true>, b, kThreads, 0, s, lam, lat, k, table, q, n, tmp);
-    else
-        launchDependent(postGatherKernel<R, false>, b, kThreads, 0, s, lam, lat, k, table, q, n, tmp);
-    if (const int rc = checkLaunch("BC adjoint gather"))
-        return rc;
+    if (tmp) {
+        if (even)
+            launchDependent(postGatherKernel<R, true>, b, kThreads, 0, s, lam, lat, k, table, q, n, tmp);
+        else
+            launchDependent(postGatherKernel<R, false>, b, kThreads, 0, s, lam, lat, k, table, q, n, tmp);
+        if (const int rc = checkLaunch("BC adjoint gather"))
+            return rc;
+    }
     constexpr int V = VFB_BC_VELOCITY_INTERPOLATED, NS = VFB_BC_NOSLIP_INTERPOLATED;
     if (kind == V)
         (even ? launchPostScatter<R, V, true> : launchPostScatter<R, V, false>)(b, s, lam, lat, k, table, q, n, rec,
@@ -761,22 +893,28 @@ int postBCAdjointLists(R* lam, const BcLattice<R>& lat, PostLists<R> P, bool eve
         return rc;
     if (b == 0)
         return VFB_OK;
-    if (even)
-        launchDependent(postGatherListsKernel<R, true>, b, kThreads, 0, s, lam, lat, P);
-    else
-        launchDependent(postGatherListsKernel<R, false>, b, kThreads, 0, s, lam, lat, P);
-    if (const int rc = checkLaunch("BC lists adjoint gather"))
-        return rc;
-    if (even)
-        launchDependent(postScatterListsKernel<R, true>, b, kThreads, 0, s, lam, lat, P);
-    else
-        launchDependent(postScatterListsKernel<R, false>, b, kThreads, 0, s, lam, lat, P);
+    if (P.list[0].tmp) {
+        if (even)
+            launchDependent(postGatherListsKernel<R, true>, b, kThreads, 0, s, lam, lat, P);
+        else
+            launchDependent(postGatherListsKernel<R, false>, b, kThreads, 0, s, lam, lat, P);
+        if (const int rc = checkLaunch("BC lists adjoint gather"))
+            return rc;
+        if (even)
+            launchDependent(postScatterListsKernel<R, true, false>, b, kThreads, 0, s, lam, lat, P);
+        else
+            launchDependent(postScatterListsKernel<R, false, false>, b, kThreads, 0, s, lam, lat, P);
+    } else if (even) {
+        launchDependent(postScatterListsKernel<R, true, true>, b, kThreads, 0, s, lam, lat, P);
+    } else {
+        launchDependent(postScatterListsKernel<R, false, true>, b, kThreads, 0, s, lam, lat, P);
+    }
     return checkLaunch("BC lists adjoint scatter");
 }
 
 template <class R>
-int pressureBC(R* dist, const BcLattice<R>& lat, const int32_t* k, const int32_t* kN, const R* rhoBC, uint32_t n,
-               int direction, bool even, R* rec, cudaStream_t s)
+int pressureBC(R* dist, const BcLattice<R>& lat, const uint32_t* table, const R* rhoBC, uint32_t n, int direction,
+               bool even, R* rec, cudaStream_t s)
 {
     if (n == 0)
         return VFB_OK;
@@ -785,15 +923,15 @@ int pressureBC(R* dist, const BcLattice<R>& lat, const int32_t* k, const int32_t
         return rc;
     const unsigned b = blocksFor(n);
     if (even)
-        launchDependent(pressureKernel<R, true>, b, kThreads, 0, s, dist, lat, k, kN, rhoBC, n, axis, sgn, rec);
+        launchDependent(pressureKernel<R, true>, b, kThreads, 0, s, dist, lat, table, rhoBC, n, axis, sgn, rec);
     else
-        launchDependent(pressureKernel<R, false>, b, kThreads, 0, s, dist, lat, k, kN, rhoBC, n, axis, sgn, rec);
+        launchDependent(pressureKernel<R, false>, b, kThreads, 0, s, dist, lat, table, rhoBC, n, axis, sgn, rec);
     return checkLaunch("adjoint forward pressure BC");
 }
 
 template <class R>
-int pressureBCAdjoint(R* lam, const BcLattice<R>& lat, const int32_t* k, const int32_t* kN, const R* rhoBC,
-                      uint32_t n, int direction, bool even, const R* rec, R* tmp, cudaStream_t s)
+int pressureBCAdjoint(R* lam, const BcLattice<R>& lat, const uint32_t* table, const R* rhoBC, uint32_t n,
+                      int direction, bool even, const R* rec, R* tmp, cudaStream_t s)
 {
     if (n == 0)
         return VFB_OK;
@@ -801,17 +939,26 @@ int pressureBCAdjoint(R* lam, const BcLattice<R>& lat, const int32_t* k, const i
     if (const int rc = axisOf(direction, axis, sgn))
         return rc;
     const unsigned b = blocksFor(n);
-    if (even)
-        launchDependent(pressureGatherKernel<R, true>, b, kThreads, 0, s, lam, lat, k, n, axis, sgn, tmp);
-    else
-        launchDependent(pressureGatherKernel<R, false>, b, kThreads, 0, s, lam, lat, k, n, axis, sgn, tmp);
-    if (const int rc = checkLaunch("pressure adjoint gather"))
-        return rc;
-    if (even)
-        launchDependent(pressureScatterKernel<R, true>, b, kThreads, 0, s, lam, lat, kN, rhoBC, n, axis, sgn, rec,
-                        tmp);
-    else
-        launchDependent(pressureScatterKernel<R, false>, b, kThreads, 0, s, lam, lat, kN, rhoBC, n, axis, sgn, rec, tmp);
+    if (tmp) {
+        if (even)
+            launchDependent(pressureGatherKernel<R, true>, b, kThreads, 0, s, lam, lat, table, n, axis, sgn, tmp);
+        else
+            launchDependent(pressureGatherKernel<R, false>, b, kThreads, 0, s, lam, lat, table, n, axis, sgn, tmp);
+        if (const int rc = checkLaunch("pressure adjoint gather"))
+            return rc;
+        if (even)
+            launchDependent(pressureScatterKernel<R, true, false>, b, kThreads, 0, s, lam, lat, table, rhoBC, n, axis,
+                            sgn, rec, tmp);
+        else
+            launchDependent(pressureScatterKernel<R, false, false>, b, kThreads, 0, s, lam, lat, table, rhoBC, n,
+                            axis, sgn, rec, tmp);
+    } else if (even) {
+        launchDependent(pressureScatterKernel<R, true, true>, b, kThreads, 0, s, lam, lat, table, rhoBC, n, axis, sgn,
+                        rec, tmp);
+    } else {
+        launchDependent(pressureScatterKernel<R, false, true>, b, kThreads, 0, s, lam, lat, table, rhoBC, n, axis,
+                        sgn, rec, tmp);
+    }
     return checkLaunch("pressure adjoint scatter");
 }
 
@@ -851,10 +998,10 @@ int reducePartials(const double* partials, unsigned blocks, int width, double* a
                                   const R*, const R*, const R*, bool, const R*, R*, double*, cudaStream_t);            \
     template int postBCLists<R>(R*, const BcLattice<R>&, PostLists<R>, bool, cudaStream_t);                          \
     template int postBCAdjointLists<R>(R*, const BcLattice<R>&, PostLists<R>, bool, cudaStream_t);                   \
-    template int pressureBC<R>(R*, const BcLattice<R>&, const int32_t*, const int32_t*, const R*, uint32_t, int,     \
-                               bool, R*, cudaStream_t);                                                                \
-    template int pressureBCAdjoint<R>(R*, const BcLattice<R>&, const int32_t*, const int32_t*, const R*, uint32_t,   \
-                                      int, bool, const R*, R*, cudaStream_t);                                          \
+    template int pressureBC<R>(R*, const BcLattice<R>&, const uint32_t*, const R*, uint32_t, int, bool, R*,          \
+                               cudaStream_t);                                                                          \
+    template int pressureBCAdjoint<R>(R*, const BcLattice<R>&, const uint32_t*, const R*, uint32_t, int, bool,       \
+                                      const R*, R*, cudaStream_t);                                                     \
     template int objective<R>(const R*, unsigned long long, const uint32_t*, const uint32_t*, const uint32_t*,       \
                               const uint32_t*, const double*, const double*, const double*, uint32_t, bool, double*,  \
                               R*, double, cudaStream_t);

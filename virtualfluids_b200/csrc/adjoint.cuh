@@ -21,7 +21,8 @@
 // Overwritten cells: a BC writes some cells without reading them, so its
 // adjoint runs in two launches: "gather" moves lam at every written cell into
 // tmp[d * n + i] and clears the cell; "scatter" adds the contributions of the
-// node's formula to the cells it read.  The entries of a list write disjoint
+// node's formula to the cells it read.  When no entry writes a cell an entry
+// reads, both run in one launch without tmp.  The entries of a list write disjoint
 // cells, so the gather does not race; the scatters add with atomics, since a
 // node may appear in a list more than once (edge nodes of two walls, each
 // entry with the directions of its wall) and two pressure nodes may share a
@@ -39,8 +40,8 @@ namespace vfb
 {
 namespace adjoint
 {
-// blocks of the collision adjoint (its block partial sums of the force adjoint)
-unsigned collisionBlocks(uint32_t nFluid);
+// partial sums of the force adjoint that the collision adjoint keeps (one per warp)
+unsigned collisionPartials(uint32_t nFluid);
 
 // forward K17 collision over the fluid list; tape may be null; loc is the
 // fluid list's location table (8 * nFluid, vfb_bc_locations layout) or null
@@ -49,8 +50,8 @@ int collision(R* dist, unsigned long long N, const uint32_t* nX, const uint32_t*
               const uint32_t* fluid, const uint32_t* loc, uint32_t nFluid, const K17Rates<R>& rates, R fx, R fy, R fz,
               bool even, R* tape, cudaStream_t s);
 
-// adjoint of the collision: lam in place; partials[3 * b + c] accumulate the
-// block sums of the adjoint of the half force (fx, fy, fz) (the caller
+// adjoint of the collision: lam in place; partials[3 * w + c] accumulate the
+// warp sums of the adjoint of the half force (fx, fy, fz) (the caller
 // clears them before the first step and reduces them after the last)
 template <class R>
 int collisionAdjoint(R* lam, unsigned long long N, const uint32_t* nX, const uint32_t* nY, const uint32_t* nZ,
@@ -64,7 +65,8 @@ template <class R>
 int postBC(int kind, R* dist, const BcLattice<R>& lat, const int32_t* k, const uint32_t* table, const R* q, uint32_t n,
            const R* Vx, const R* Vy, const R* Vz, bool even, R* rec, cudaStream_t s);
 
-// adjoint of postBC: gather then scatter; gV (3 n doubles: x block, y block,
+// adjoint of postBC: gather then scatter, or both in one launch with tmp null
+// (no entry of the step's lists writes a cell an entry reads); gV (3 n doubles: x block, y block,
 // z block) accumulates the adjoint of the BC velocities (velocity kind)
 template <class R>
 int postBCAdjoint(int kind, R* lam, const BcLattice<R>& lat, const int32_t* k, const uint32_t* table, const R* q,
@@ -100,14 +102,16 @@ template <class R>
 int postBCLists(R* dist, const BcLattice<R>& lat, PostLists<R> lists, bool even, cudaStream_t s);
 template <class R>
 int postBCAdjointLists(R* lam, const BcLattice<R>& lat, PostLists<R> lists, bool even, cudaStream_t s);
-// forward non-equilibrium pressure BC (after the swap); rec may be null
+// forward non-equilibrium pressure BC (after the swap); rec may be null; table
+// holds the list's locations (16 n: the nodes' eight, then the neighbours')
 template <class R>
-int pressureBC(R* dist, const BcLattice<R>& lat, const int32_t* k, const int32_t* kN, const R* rhoBC, uint32_t n,
-               int direction, bool even, R* rec, cudaStream_t s);
+int pressureBC(R* dist, const BcLattice<R>& lat, const uint32_t* table, const R* rhoBC, uint32_t n, int direction,
+               bool even, R* rec, cudaStream_t s);
 
+// its adjoint; tmp null: in one launch (no entry's neighbour is an entry's node)
 template <class R>
-int pressureBCAdjoint(R* lam, const BcLattice<R>& lat, const int32_t* k, const int32_t* kN, const R* rhoBC,
-                      uint32_t n, int direction, bool even, const R* rec, R* tmp, cudaStream_t s);
+int pressureBCAdjoint(R* lam, const BcLattice<R>& lat, const uint32_t* table, const R* rhoBC, uint32_t n,
+                      int direction, bool even, const R* rec, R* tmp, cudaStream_t s);
 
 // objective J = sum_j wx_j ux + wy_j uy + wz_j uz over nodes[j], u = j / (1 +
 // drho) of the populations of parity `even`: block partials of J into

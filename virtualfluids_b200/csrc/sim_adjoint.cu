@@ -48,7 +48,7 @@ struct AdjointState {
     std::vector<size_t> pressureOffset; // first entry of each pressure list in recPressure / tmpPressure
     size_t pressureTotal = 0;
     DeviceBuffer objNodes, objW[3], partials, accForce, gVelocity;
-    DeviceBuffer forcePartials; // 3 per collision block, accumulated over a backward pass
+    DeviceBuffer forcePartials; // 3 per collision warp, accumulated over a backward pass
     DeviceBuffer fluidLocations; // 8 * nFluid: the fluid list's node locations (vfb_bc_locations)
     uint32_t nObj = 0;
     int velocityKind = -1, noSlipKind = -1, geometryKind = -1;
@@ -56,6 +56,10 @@ struct AdjointState {
     // the post-collision lists write cells no other list reads or writes, so
     // each step launches them together (-1: not checked yet)
     int listsCommute = -1;
+    // no entry of the post-collision lists writes a cell an entry reads, so
+    // their adjoints gather and scatter in one launch; the same per pressure list
+    bool listsFused = false;
+    std::vector<char> pressureFused;
     // the forward pass recorded the tapes and BC records of its only segment:
     // the backward pass reverses them without recomputing the steps
     bool taped = false;
@@ -215,8 +219,8 @@ struct Stepper {
                     continue;
                 R* rec = slot < 0 ? nullptr : as<R>(A.recPressure) + (size_t)slot * 27 * A.pressureTotal +
                                                   27 * A.pressureOffset[p];
-                if (const int rc = adjoint::pressureBC<R>(dist, t, as<const int32_t>(P.k), as<const int32_t>(P.kN),
-                                                          as<const R>(P.rho), P.n, P.direction, even, rec, s))
+                if (const int rc = adjoint::pressureBC<R>(dist, t, as<const uint32_t>(P.locations), as<const R>(P.rho),
+                                                          P.n, P.direction, even, rec, s))
                     return rc;
             }
         return VFB_OK;
@@ -233,9 +237,10 @@ struct Stepper {
                     continue;
                 const size_t off = 27 * A.pressureOffset[p];
                 const R* rec = as<R>(A.recPressure) + (size_t)slot * 27 * A.pressureTotal + off;
-                if (const int rc = adjoint::pressureBCAdjoint<R>(lam, lat, as<const int32_t>(P.k),
-                                                                 as<const int32_t>(P.kN), as<const R>(P.rho), P.n,
-                                                                 P.direction, !even, rec, as<R>(A.tmpPressure) + off,
+                if (const int rc = adjoint::pressureBCAdjoint<R>(lam, lat, as<const uint32_t>(P.locations),
+                                                                 as<const R>(P.rho), P.n, P.direction, !even, rec,
+                                                                 A.pressureFused[p] ? nullptr
+                                                                                    : as<R>(A.tmpPressure) + off,
                                                                  s))
                     return rc;
             }
@@ -252,8 +257,8 @@ struct Stepper {
             adjoint::PostLists<R> P;
             for (Item& it : items)
                 if (it.list->n && it.kind >= 0)
-                    P.list[P.count++] = postList(*it.list, it.kind, slotOf(*it.rec, slot, it.list->n), as<R>(*it.tmp),
-                                                 it.gV);
+                    P.list[P.count++] = postList(*it.list, it.kind, slotOf(*it.rec, slot, it.list->n),
+                                                 A.listsFused ? nullptr : as<R>(*it.tmp), it.gV);
             if (const int rc = adjoint::postBCAdjointLists<R>(lam, lat, P, even, s))
                 return rc;
         }
@@ -264,7 +269,7 @@ struct Stepper {
                     it.kind, lam, lat, as<const int32_t>(it.list->k), as<const uint32_t>(it.list->locations),
                     as<const R>(it.list->q), it.list->n,
                     as<const R>(it.list->vx), as<const R>(it.list->vy), as<const R>(it.list->vz), even,
-                    slotOf(*it.rec, slot, it.list->n), as<R>(*it.tmp), it.gV, s))
+                    slotOf(*it.rec, slot, it.list->n), A.listsFused ? nullptr : as<R>(*it.tmp), it.gV, s))
                 return rc;
         }
         return adjoint::collisionAdjoint<R>(lam, L.N, nX(), nY(), nZ(), as<const uint32_t>(L.fluid),
@@ -298,15 +303,19 @@ int objectiveValue(vfb_simulation& S, AdjointState& A, const R* dist, bool even,
 }
 
 // Whether the post-collision lists of the adjoint (velocity, no-slip,
-// geometry) can run in one launch per step: in both parities, no cell a list
-// writes (the cell of inv(d) in the other view, for each link d with
-// 0 <= q_d <= 1) is written by another list or is one of the 27 cells
+// geometry) can run in one launch per step (commute): in both parities, no
+// cell a list writes (the cell of inv(d) in the other view, for each link d
+// with 0 <= q_d <= 1) is written by another list or is one of the 27 cells
 // another list's nodes read.  Then the lists commute, forward and adjoint.
-// VFB_ADJOINT_SEPARATE_LISTS=1 keeps one launch per list (for comparisons).
+// And whether the adjoint's gather and scatter can (fused): no cell any entry
+// writes is read by an entry, of its own list or another, and no two lists
+// write one cell.
+// VFB_ADJOINT_SEPARATE_LISTS=1 keeps one launch per list and separate gathers
+// (for comparisons).
 template <class R>
-int listsCommute(vfb_simulation& S, AdjointState& A, cudaStream_t s, bool& result)
+int listsCommute(vfb_simulation& S, AdjointState& A, cudaStream_t s, bool& commute, bool& fused)
 {
-    result = false;
+    commute = fused = false;
     if (const char* env = std::getenv("VFB_ADJOINT_SEPARATE_LISTS"))
         if (env[0] == '1')
             return VFB_OK;
@@ -332,8 +341,8 @@ int listsCommute(vfb_simulation& S, AdjointState& A, cudaStream_t s, bool& resul
     }
     if (cudaStreamSynchronize(s) != cudaSuccess)
         return cudaFail("BC list download");
-    if (locs.size() < 2)
-        return VFB_OK; // nothing to launch together
+    commute = locs.size() > 1; // else nothing to launch together
+    fused = true;
     const unsigned long long N = L.N;
     for (int parity = 0; parity < 2; ++parity) {
         const bool even = parity == 0;
@@ -350,7 +359,7 @@ int listsCommute(vfb_simulation& S, AdjointState& A, cudaStream_t s, bool& resul
                         (unsigned long long)(even ? slot<false>(e) : slot<true>(e)) * N + locs[l][(size_t)loc(e) * n + i];
                     const auto ins = written.emplace(c, (int)l);
                     if (!ins.second && ins.first->second != (int)l)
-                        return VFB_OK; // two lists write one cell
+                        commute = fused = false; // two lists write one cell
                 }
         }
         for (size_t l = 0; l < locs.size(); ++l) {
@@ -361,12 +370,44 @@ int listsCommute(vfb_simulation& S, AdjointState& A, cudaStream_t s, bool& resul
                     const unsigned long long c =
                         (unsigned long long)(even ? slot<true>(r) : slot<false>(r)) * N + locs[l][(size_t)loc(r) * n + i];
                     const auto it = written.find(c);
-                    if (it != written.end() && it->second != (int)l)
-                        return VFB_OK; // a list reads a cell another list writes
+                    if (it == written.end())
+                        continue;
+                    fused = false; // an entry reads a cell an entry writes
+                    if (it->second != (int)l)
+                        commute = false; // a list reads a cell another list writes
                 }
         }
+        if (!fused && !commute)
+            return VFB_OK;
     }
-    result = true;
+    return VFB_OK;
+}
+
+// per pressure list: whether its adjoint can gather and scatter in one launch.
+// The gather clears cells of the list's nodes and the scatter adds to cells of
+// their neighbours; every cell of one view belongs to one node, so it can when
+// no neighbour is a node of the list.
+int pressureFused(vfb_simulation& S, AdjointState& A, cudaStream_t s)
+{
+    Level& L = *S.levels[0];
+    A.pressureFused.assign(L.pressure.size(), 0);
+    if (const char* env = std::getenv("VFB_ADJOINT_SEPARATE_LISTS"))
+        if (env[0] == '1')
+            return VFB_OK;
+    for (size_t p = 0; p < L.pressure.size(); ++p) {
+        const PressureListDevice& P = *L.pressure[p];
+        std::vector<int32_t> k(P.n), kN(P.n);
+        if (P.n && (cudaMemcpyAsync(k.data(), P.k.ptr, P.n * sizeof(int32_t), cudaMemcpyDeviceToHost, s) ||
+                    cudaMemcpyAsync(kN.data(), P.kN.ptr, P.n * sizeof(int32_t), cudaMemcpyDeviceToHost, s) ||
+                    cudaStreamSynchronize(s)))
+            return cudaFail("pressure list download");
+        std::sort(k.begin(), k.end());
+        char fused = 1;
+        for (const int32_t n : kN)
+            if (std::binary_search(k.begin(), k.end(), n))
+                fused = 0;
+        A.pressureFused[p] = fused;
+    }
     return VFB_OK;
 }
 
@@ -392,7 +433,7 @@ int ensureSegmentBuffers(vfb_simulation& S, AdjointState& A)
         once(A.tmpVelocity, L.velocity.n) || once(A.tmpNoSlip, L.noSlip.n) || once(A.tmpGeometry, L.geometry.n) ||
         once(A.tmpPressure, A.pressureTotal) ||
         ensure(A.gVelocity, std::max<size_t>(1, 3ull * L.velocity.n * sizeof(double))) ||
-        ensure(A.forcePartials, 3ull * std::max(1u, adjoint::collisionBlocks(L.nFluid)) * sizeof(double)))
+        ensure(A.forcePartials, 3ull * std::max(1u, adjoint::collisionPartials(L.nFluid)) * sizeof(double)))
         return cudaFail("adjoint buffers");
     for (size_t i = 0; i < before.size(); ++i)
         if (held[i]->ptr != before[i]) {
@@ -426,7 +467,9 @@ int adjointForward(vfb_simulation& S, AdjointState& A, unsigned steps, double* J
     }
     if (A.listsCommute < 0) {
         bool ok = false;
-        if (const int rc = listsCommute<R>(S, A, s, ok))
+        if (const int rc = listsCommute<R>(S, A, s, ok, A.listsFused))
+            return rc;
+        if (const int rc = pressureFused(S, A, s))
             return rc;
         A.listsCommute = ok ? 1 : 0;
     }
@@ -530,7 +573,7 @@ int adjointBackward(vfb_simulation& S, AdjointState& A, double seed, double* dVe
             return cudaFail("segment graph launch");
     }
     // the force adjoint: every block's sum over all steps, reduced once in block order
-    if (const int rc = adjoint::reducePartials(as<double>(A.forcePartials), adjoint::collisionBlocks(L.nFluid), 3,
+    if (const int rc = adjoint::reducePartials(as<double>(A.forcePartials), adjoint::collisionPartials(L.nFluid), 3,
                                                as<double>(A.accForce), 0.5 * L.forceFactor, s))
         return rc;
     if (dVelocity && L.velocity.n &&
@@ -664,7 +707,7 @@ extern "C" int vfb_sim_adjoint_forward(vfb_simulation* sim, unsigned int steps, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     A.nObj = numberOfObjectiveNodes;
     const size_t n = std::max<uint32_t>(1, numberOfObjectiveNodes);
-    const unsigned partials = std::max(adjoint::collisionBlocks(L.nFluid), adjoint::objectiveBlocks(A.nObj));
+    const unsigned partials = std::max(adjoint::collisionPartials(L.nFluid), adjoint::objectiveBlocks(A.nObj));
     if (ensure(A.objNodes, n * sizeof(uint32_t)) || ensure(A.objW[0], n * sizeof(double)) ||
         ensure(A.objW[1], n * sizeof(double)) || ensure(A.objW[2], n * sizeof(double)) ||
         ensure(A.partials, 3ull * std::max(1u, partials) * sizeof(double)) || ensure(A.accForce, 4 * sizeof(double)))
