@@ -225,6 +225,19 @@ __device__ __forceinline__ void collideNode(const TiledArgs<S>& a, typename Stor
     }
 }
 
+// The tile of a block of the direct and paired kernels: ascending in the even
+// steps, descending in the odd ones, so that a step starts on the tiles the
+// previous one ended with, whose populations are still in L2 (126 MB).  B200,
+// pairs of steps that alternate between three lattices: FP64 128^3 (0.45 GB)
+// 367 -> 345 us, BGK FP32 on 219 x 187 x 133 (0.59 GB) 438 -> 426 us, FP16
+// 192^3 (0.38 GB) 474 -> 466 us, FP32 256^3 (1.8 GB) 1326 -> 1320 us.
+template <class S, bool EVEN>
+__device__ __forceinline__ uint32_t tileOf(const TiledArgs<S>& a)
+{
+    const uint32_t t = blockIdx.x - a.laneBlocks;
+    return EVEN ? t : a.nTiles - 1 - t;
+}
+
 // entry i of the plan's lane list, through its location table
 template <class S, bool EVEN, Op OP, bool WM, bool BF>
 __device__ __forceinline__ void collideLane(const TiledArgs<S>& a, uint32_t i)
@@ -388,7 +401,7 @@ __global__ void __launch_bounds__(C::T, C::MINB) directKernel(const TiledArgs<S>
         return;
     }
     const int warp = tid >> 5, lane = tid & 31;
-    const uint32_t* meta = a.meta + (size_t)(blockIdx.x - a.laneBlocks) * C::META_WORDS;
+    const uint32_t* meta = a.meta + (size_t)tileOf<S, EVEN>(a) * C::META_WORDS;
     const bool active = (__ldg(meta + 4 + warp) >> lane) & 1u;
     if (!active)
         return;
@@ -448,7 +461,7 @@ __global__ void __launch_bounds__(C::T / 2, C::MINB) pairKernel(const TiledArgs<
         collideLane<S, EVEN, OP, WM, BF>(a, blockIdx.x * HALF + tid);
         return;
     }
-    const uint32_t tile = blockIdx.x - a.laneBlocks;
+    const uint32_t tile = tileOf<S, EVEN>(a);
     const uint32_t* meta = a.meta + (size_t)tile * C::META_WORDS;
     const uint32_t maskA = __ldg(meta + 4 + warp), maskB = __ldg(meta + 4 + W2 + warp);
     const bool actA = (maskA >> lane) & 1u;
