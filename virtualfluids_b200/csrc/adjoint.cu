@@ -49,6 +49,17 @@ constexpr int kAdjointBlocksFP64 = 2;
 
 unsigned blocksFor(uint32_t n) { return (n + kThreads - 1) / kThreads; }
 
+// The part of the fluid list a block takes: ascending in the steps of even
+// parity, descending in the others, so that a step starts on the populations
+// the previous one left in L2.  The tape passes by with streaming accesses
+// (read and written once a pass), so that it does not displace them (channel
+// 128 x 64 x 64, per step: FP32 188 -> 177 us, FP64 291 -> 280 us).
+template <bool EVEN>
+__device__ __forceinline__ uint32_t partOf()
+{
+    return EVEN ? blockIdx.x : gridDim.x - 1 - blockIdx.x;
+}
+
 template <class R>
 __device__ __forceinline__ unsigned long long cell(int slotIndex, unsigned long long N, uint32_t location)
 {
@@ -115,7 +126,7 @@ __global__ void __launch_bounds__(kThreads)
                         const K17Rates<R> r, R fx, R fy, R fz, R* __restrict__ tape)
 {
     gridDependencyWait();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = partOf<EVEN>() * kThreads + threadIdx.x;
     if (i >= n)
         return;
     const Locs L = fluidLocations(table, i, n, fluid, nX, nY, nZ);
@@ -126,7 +137,7 @@ __global__ void __launch_bounds__(kThreads)
     if (tape) {
 #pragma unroll
         for (int d = 0; d < 27; ++d)
-            tape[(unsigned long long)d * n + i] = f[d];
+            __stcs(tape + (unsigned long long)d * n + i, f[d]);
     }
     R drho, ux, uy, uz;
     k17Collide<R>(f, r, fx, fy, fz, drho, ux, uy, uz);
@@ -146,7 +157,7 @@ __global__ void __launch_bounds__(kThreads, 4)
                             uint32_t n, const K17Rates<F2> r, float fx, float fy, float fz, float* __restrict__ tape)
 {
     gridDependencyWait();
-    const uint32_t i = blockIdx.x * (2 * kThreads) + threadIdx.x;
+    const uint32_t i = partOf<EVEN>() * (2 * kThreads) + threadIdx.x;
     if (i >= n)
         return;
     const bool both = i + kThreads < n;
@@ -169,9 +180,9 @@ __global__ void __launch_bounds__(kThreads, 4)
 #pragma unroll
         for (int d = 0; d < 27; ++d) {
             float* p = tape + (unsigned long long)d * n;
-            p[i] = f[d].v.x;
+            __stcs(p + i, f[d].v.x);
             if (both)
-                p[j] = f[d].v.y;
+                __stcs(p + j, f[d].v.y);
         }
     }
     F2 drho, ux, uy, uz;
@@ -204,14 +215,14 @@ __global__ void __launch_bounds__(kThreads, MINB)
                            double* __restrict__ partials)
 {
     gridDependencyWait();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = partOf<EVEN>() * kThreads + threadIdx.x;
     double gx = 0.0, gy = 0.0, gz = 0.0;
     if (i < n) {
         const Locs L = fluidLocations(table, i, n, fluid, nX, nY, nZ);
         R a[27], l[27];
 #pragma unroll
         for (int d = 0; d < 27; ++d)
-            a[d] = tape[(unsigned long long)d * n + i];
+            a[d] = __ldcs(tape + (unsigned long long)d * n + i);
 #pragma unroll
         for (int d = 0; d < 27; ++d)
             l[inv(d)] = lam[cell<R>(slot<EVEN>(d), N, L.k[loc(d)])];
