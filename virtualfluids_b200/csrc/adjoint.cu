@@ -404,7 +404,7 @@ __device__ __forceinline__ void postScatterEntry(R* lam, const BcLattice<R>& lat
         const int e = inv(d);
         const R t = tv[j];
         const R w = weight<R>(d);
-        const R r = linkReciprocal(R(1) + qd);
+        const R r = reciprocal(R(1) + qd);
         const R A = (R(1) - qd) * r;
         const R b = qd * r;
         gg[d] += t * (A * R(0.5) * (R(1) + c1) + b);

@@ -44,20 +44,6 @@ __device__ __forceinline__ void bcMacros(const R* g, R& drho, R& vx1, R& vx2, R&
     vx3 = pyramidJz(g) * oneOverRho;
 }
 
-// 1 / (1 + q) of a link, q in [0, 1]: in FP64 the single-precision reciprocal
-// and two Newton-Raphson steps r (2 - x r), instead of a division per link
-__device__ __forceinline__ float linkReciprocal(float x) { return reciprocal(x); }
-__device__ __forceinline__ double linkReciprocal(double x)
-{
-#ifdef __CUDA_ARCH__
-    double r = (double)approximateReciprocal((float)x);
-    r = fma(fma(-x, r, 1.0), r, r);
-    return fma(fma(-x, r, 1.0), r, r);
-#else
-    return 1.0 / x;
-#endif
-}
-
 // KernelUtilities.h:171-174
 template <class R>
 __device__ __forceinline__ R feqBC(R drho, R vel, R cuSq, R w)
@@ -73,9 +59,9 @@ struct LinkRates {
 };
 
 // KernelUtilities.h:176-195: the interpolated bounce-back of a link with wall
-// distance q, over the common denominator 1 + q (one reciprocal a link, where
-// the formula as written has three divisions; those were most of an FP64
-// list's time, and the chain that a short list waits for):
+// distance q, over the common denominator 1 + q (one reciprocal a link, by
+// Newton-Raphson steps, where the formula as written has three divisions; those
+// were most of an FP64 list's time, and the chain that a short list waits for):
 //   [ (1 - q) / 2 (f - finv + (f + finv - 2 omega feq) / (1 - omega)) + q (f + finv) - moving ] / (1 + q)
 // moving: 6 w c.u of a moving wall, 0 of one at rest
 template <class R>
@@ -83,7 +69,7 @@ __device__ __forceinline__ R interpolatedLink(R q, R f, R finv, R feq, const Lin
 {
     const R s = f + finv;
     const R t = fma(fma(-r.twoOmega, feq, s), r.inverse, f - finv);
-    return fma(fma(R(-0.5), q, R(0.5)), t, fma(q, s, -moving)) * linkReciprocal(R(1) + q);
+    return fma(fma(R(-0.5), q, R(0.5)), t, fma(q, s, -moving)) * reciprocal(R(1) + q);
 }
 
 template <class R>

@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(128) bcStressKernel(S* __restrict__ dist, cons
         const int e = inv(d);
         R term = R(6) * weight<R>(d) * cdot<R>(d, V[0], V[1], V[2]);
         if (KIND == VFB_BC_STRESS_INTERPOLATED)
-            term = term * linkReciprocal(R(1) + qv[j]);
+            term = term * reciprocal(R(1) + qv[j]);
         Storage<S>::store(dist + (unsigned long long)slot<!EVEN>(e) * N + L.k[loc(e)], fin[j] - term, d);
         if (cx(d) > 0) mom[0] = mom[0] - term; else if (cx(d) < 0) mom[0] = mom[0] + term;
         if (cy(d) > 0) mom[1] = mom[1] - term; else if (cy(d) < 0) mom[1] = mom[1] + term;
