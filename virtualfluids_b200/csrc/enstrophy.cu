@@ -10,9 +10,11 @@
 // block, like the mass / energy sums.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "capi_common.cuh"
+#include "output.hpp"
 #include "d3q27.cuh"
 
 namespace vfb
@@ -148,6 +150,43 @@ void nodesOnHost(const void* rho, const void* vx, const void* vy, const void* vz
     }
 }
 } // namespace
+
+unsigned enstrophyBlocks(unsigned long long N)
+{
+    int device = 0, sms = 148;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const unsigned long long need = (N + kEnstrophyThreads - 1) / kEnstrophyThreads;
+    return (unsigned)std::min<unsigned long long>((unsigned long long)sms * 4u, need);
+}
+
+int enstrophyLaunch(int precision, const void* rho, const void* vx, const void* vy, const void* vz,
+                    unsigned long long N, const uint32_t* geo, const uint32_t* nX, const uint32_t* nY,
+                    const uint32_t* nZ, const uint32_t* neighborInverse, double* partial, cudaStream_t s)
+{
+    const unsigned blocks = enstrophyBlocks(N);
+    const AxisWalk walk { nX, nY, nZ, neighborInverse };
+    if (precision == VFB_FP64)
+        enstrophyKernel<double><<<blocks, kEnstrophyThreads, 0, s>>>(
+            static_cast<const double*>(rho), static_cast<const double*>(vx), static_cast<const double*>(vy),
+            static_cast<const double*>(vz), N, geo, walk, partial);
+    else
+        enstrophyKernel<float><<<blocks, kEnstrophyThreads, 0, s>>>(
+            static_cast<const float*>(rho), static_cast<const float*>(vx), static_cast<const float*>(vy),
+            static_cast<const float*>(vz), N, geo, walk, partial);
+    return checkLaunch("enstrophy");
+}
+
+void enstrophyMean(const double* partial, unsigned blocks, double* out2)
+{
+    double sum = 0.0, count = 0.0;
+    for (unsigned b = 0; b < blocks; ++b) {
+        sum += partial[2 * b + 0];
+        count += partial[2 * b + 1];
+    }
+    out2[0] = count > 0.0 ? sum / count : 0.0;
+    out2[1] = count;
+}
 } // namespace vfb
 
 using namespace vfb;
@@ -167,26 +206,11 @@ extern "C" int vfb_enstrophy(int precision, const void* rho, const void* vx, con
     if (precision != VFB_FP64 && precision != VFB_FP32)
         return setError(VFB_ERR_INVALID_ARGUMENT, "precision must be VFB_FP64 or VFB_FP32");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int device = 0, sms = 148;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    unsigned blocks = (unsigned)sms * 4u;
-    const unsigned long long need = (N + kEnstrophyThreads - 1) / kEnstrophyThreads;
-    if (need < blocks)
-        blocks = (unsigned)need;
+    const unsigned blocks = enstrophyBlocks(N);
     double* partial = nullptr;
     if (cudaMallocAsync(&partial, sizeof(double) * 2 * blocks, s) != cudaSuccess)
         return setError(VFB_ERR_CUDA, "cudaMallocAsync of %u partial sums failed", blocks);
-    const AxisWalk walk { nX, nY, nZ, neighborInverse };
-    if (precision == VFB_FP64)
-        enstrophyKernel<double><<<blocks, kEnstrophyThreads, 0, s>>>(
-            static_cast<const double*>(rho), static_cast<const double*>(vx), static_cast<const double*>(vy),
-            static_cast<const double*>(vz), N, geo, walk, partial);
-    else
-        enstrophyKernel<float><<<blocks, kEnstrophyThreads, 0, s>>>(
-            static_cast<const float*>(rho), static_cast<const float*>(vx), static_cast<const float*>(vy),
-            static_cast<const float*>(vz), N, geo, walk, partial);
-    int rc = checkLaunch("enstrophy");
+    int rc = enstrophyLaunch(precision, rho, vx, vy, vz, N, geo, nX, nY, nZ, neighborInverse, partial, s);
     if (rc == VFB_OK) {
         std::vector<double> host(2 * (size_t)blocks);
         if (cudaMemcpyAsync(host.data(), partial, sizeof(double) * 2 * blocks, cudaMemcpyDeviceToHost, s) !=
@@ -194,13 +218,7 @@ extern "C" int vfb_enstrophy(int precision, const void* rho, const void* vx, con
             cudaStreamSynchronize(s) != cudaSuccess) {
             rc = setError(VFB_ERR_CUDA, "copy of partial sums failed: %s", cudaGetErrorString(cudaGetLastError()));
         } else {
-            double sum = 0.0, count = 0.0;
-            for (unsigned b = 0; b < blocks; ++b) {
-                sum += host[2 * b + 0];
-                count += host[2 * b + 1];
-            }
-            out2[0] = count > 0.0 ? sum / count : 0.0;
-            out2[1] = count;
+            enstrophyMean(host.data(), blocks, out2);
         }
     }
     cudaFreeAsync(partial, s);

@@ -13,11 +13,13 @@
 // on the fields this one wrote.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "capi_common.cuh"
 #include "collision_math.cuh"
 #include "d3q27.cuh"
+#include "output.hpp"
 #include "storage.cuh"
 
 namespace vfb
@@ -112,6 +114,39 @@ int launchOutput(const void* dist, unsigned long long N, const uint32_t* geo, co
     return checkLaunch("output pass");
 }
 } // namespace
+
+unsigned outputBlocks(unsigned long long N)
+{
+    int device = 0, sms = 148;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const unsigned long long need = (N + kOutThreads - 1) / kOutThreads;
+    return (unsigned)std::min<unsigned long long>((unsigned long long)sms * 8u, need);
+}
+
+int outputLaunch(int storage, const void* dist, unsigned long long N, const uint32_t* geo, const uint32_t* nX,
+                 const uint32_t* nY, const uint32_t* nZ, const uint8_t* mask, int even, void* rho, void* vx, void* vy,
+                 void* vz, double* partial, cudaStream_t s)
+{
+    const unsigned blocks = outputBlocks(N);
+    switch (storage) {
+    case VFB_FP32: return launchOutput<float>(dist, N, geo, nX, nY, nZ, mask, even, rho, vx, vy, vz, partial, blocks, s);
+    case VFB_FP64: return launchOutput<double>(dist, N, geo, nX, nY, nZ, mask, even, rho, vx, vy, vz, partial, blocks, s);
+    case VFB_FP16: return launchOutput<__half>(dist, N, geo, nX, nY, nZ, mask, even, rho, vx, vy, vz, partial, blocks, s);
+    case VFB_FX16: return launchOutput<int16_t>(dist, N, geo, nX, nY, nZ, mask, even, rho, vx, vy, vz, partial, blocks, s);
+    case VFB_FX16W: return launchOutput<fx16w_t>(dist, N, geo, nX, nY, nZ, mask, even, rho, vx, vy, vz, partial, blocks, s);
+    default: return launchOutput<__nv_bfloat16>(dist, N, geo, nX, nY, nZ, mask, even, rho, vx, vy, vz, partial, blocks, s);
+    }
+}
+
+void outputSums(const double* partial, unsigned blocks, double* out5)
+{
+    for (int i = 0; i < kSums; ++i)
+        out5[i] = 0.0;
+    for (unsigned b = 0; b < blocks; ++b)
+        for (int i = 0; i < kSums; ++i)
+            out5[i] += partial[(size_t)kSums * b + i];
+}
 } // namespace vfb
 
 using namespace vfb;
@@ -132,25 +167,12 @@ extern "C" int vfb_output_pass(int storage, const void* distributions, unsigned 
     if (vfb_storage_bytes(storage) == 0)
         return setError(VFB_ERR_INVALID_ARGUMENT, "unknown storage %d", storage);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int device = 0, sms = 148;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    unsigned blocks = (unsigned)sms * 8u;
-    const unsigned long long need = (N + kOutThreads - 1) / kOutThreads;
-    if (need < blocks)
-        blocks = (unsigned)need;
+    const unsigned blocks = outputBlocks(N);
     double* partial = nullptr;
     if (cudaMallocAsync(&partial, sizeof(double) * kSums * blocks, s) != cudaSuccess)
         return setError(VFB_ERR_CUDA, "cudaMallocAsync of %u partial sums failed", blocks);
     int rc = VFB_OK;
-    switch (storage) {
-    case VFB_FP32: rc = launchOutput<float>(distributions, N, geo, nX, nY, nZ, nodeMask, isEven, rho, vx, vy, vz, partial, blocks, s); break;
-    case VFB_FP64: rc = launchOutput<double>(distributions, N, geo, nX, nY, nZ, nodeMask, isEven, rho, vx, vy, vz, partial, blocks, s); break;
-    case VFB_FP16: rc = launchOutput<__half>(distributions, N, geo, nX, nY, nZ, nodeMask, isEven, rho, vx, vy, vz, partial, blocks, s); break;
-    case VFB_FX16: rc = launchOutput<int16_t>(distributions, N, geo, nX, nY, nZ, nodeMask, isEven, rho, vx, vy, vz, partial, blocks, s); break;
-    case VFB_FX16W: rc = launchOutput<fx16w_t>(distributions, N, geo, nX, nY, nZ, nodeMask, isEven, rho, vx, vy, vz, partial, blocks, s); break;
-    default: rc = launchOutput<__nv_bfloat16>(distributions, N, geo, nX, nY, nZ, nodeMask, isEven, rho, vx, vy, vz, partial, blocks, s); break;
-    }
+    rc = outputLaunch(storage, distributions, N, geo, nX, nY, nZ, nodeMask, isEven, rho, vx, vy, vz, partial, s);
     if (rc == VFB_OK) {
         std::vector<double> host((size_t)kSums * blocks);
         if (cudaMemcpyAsync(host.data(), partial, sizeof(double) * kSums * blocks, cudaMemcpyDeviceToHost, s) !=
@@ -158,9 +180,7 @@ extern "C" int vfb_output_pass(int storage, const void* distributions, unsigned 
             cudaStreamSynchronize(s) != cudaSuccess) {
             rc = setError(VFB_ERR_CUDA, "copy of partial sums failed: %s", cudaGetErrorString(cudaGetLastError()));
         } else {
-            for (unsigned b = 0; b < blocks; ++b)
-                for (int i = 0; i < kSums; ++i)
-                    out5[i] += host[(size_t)kSums * b + i];
+            outputSums(host.data(), blocks, out5);
         }
     }
     cudaFreeAsync(partial, s);

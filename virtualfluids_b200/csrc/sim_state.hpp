@@ -97,6 +97,7 @@ struct Level {
     // and kept, so repeated transfers pay no allocation)
     DeviceBuffer fields[4];
     DeviceBuffer outMask; // the output pass's node mask (built at its first call)
+    DeviceBuffer outPartials; // its and the enstrophy's partial sums
     cudaError_t fieldBuffers(size_t bytes)
     {
         for (auto& f : fields)

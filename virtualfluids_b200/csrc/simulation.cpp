@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "capi_common.cuh"
+#include "output.hpp"
 #include "sim_state.hpp"
 
 namespace vfb
@@ -1117,33 +1118,39 @@ extern "C" int vfb_sim_output(vfb_simulation* sim, int level, double* out8, void
     const auto* nX = static_cast<const uint32_t*>(L->nX.ptr);
     const auto* nY = static_cast<const uint32_t*>(L->nY.ptr);
     const auto* nZ = static_cast<const uint32_t*>(L->nZ.ptr);
-    double sums[5];
-    int rc = vfb_output_pass(sim->params.storage, L->dist.ptr, L->N, geo, nX, nY, nZ,
-                             static_cast<const uint8_t*>(L->outMask.ptr), L->isEven ? 1 : 0, f[0].ptr, f[1].ptr,
-                             f[2].ptr, f[3].ptr, sums, stream);
+    // both kernels, then the copies, then one wait: as separate calls each
+    // allocated its partial sums and waited for them (0.5 ms of an output call)
+    const unsigned blocks = outputBlocks(L->N), eBlocks = L->nNeg.ptr ? enstrophyBlocks(L->N) : 0;
+    std::vector<double> partials(5ull * blocks + 2ull * eBlocks);
+    if (!L->outPartials.ptr && L->outPartials.allocate(partials.size() * sizeof(double)) != cudaSuccess)
+        return setError(VFB_ERR_CUDA, "partial sums: %s", cudaGetErrorString(cudaGetLastError()));
+    double* const dSums = static_cast<double*>(L->outPartials.ptr);
+    int rc = outputLaunch(sim->params.storage, L->dist.ptr, L->N, geo, nX, nY, nZ,
+                          static_cast<const uint8_t*>(L->outMask.ptr), L->isEven ? 1 : 0, f[0].ptr, f[1].ptr, f[2].ptr,
+                          f[3].ptr, dSums, s);
+    if (rc == VFB_OK && eBlocks)
+        rc = enstrophyLaunch(dbl ? VFB_FP64 : VFB_FP32, f[0].ptr, f[1].ptr, f[2].ptr, f[3].ptr, L->N, geo, nX, nY, nZ,
+                             static_cast<const uint32_t*>(L->nNeg.ptr), dSums + 5ull * blocks, s);
     if (rc)
         return rc;
+    void* out[4] = { rho, vx, vy, vz };
+    for (int i = 0; i < 4; ++i)
+        if (out[i] && cudaMemcpyAsync(out[i], f[i].ptr, bytes, cudaMemcpyDeviceToHost, s) != cudaSuccess)
+            return setError(VFB_ERR_CUDA, "field copy failed");
+    if (cudaMemcpyAsync(partials.data(), dSums, partials.size() * sizeof(double), cudaMemcpyDeviceToHost, s) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        return setError(VFB_ERR_CUDA, "output: %s", cudaGetErrorString(cudaGetLastError()));
+    double sums[5];
+    outputSums(partials.data(), blocks, sums);
     out8[0] = sums[0];
     out8[1] = sums[1];
     out8[2] = sums[2];
     out8[3] = L->nEnergy ? sums[3] / (double)L->nEnergy : 0.0;
     out8[4] = (double)L->nEnergy;
     out8[7] = (double)L->nFluid;
-    if (L->nNeg.ptr) {
-        double e[2];
-        rc = vfb_enstrophy(dbl ? VFB_FP64 : VFB_FP32, f[0].ptr, f[1].ptr, f[2].ptr, f[3].ptr, L->N, geo, nX, nY, nZ,
-                           static_cast<const uint32_t*>(L->nNeg.ptr), e, stream);
-        if (rc)
-            return rc;
-        out8[5] = e[0];
-        out8[6] = e[1];
-    }
-    void* out[4] = { rho, vx, vy, vz };
-    for (int i = 0; i < 4; ++i)
-        if (out[i] && cudaMemcpyAsync(out[i], f[i].ptr, bytes, cudaMemcpyDeviceToHost, s) != cudaSuccess)
-            return setError(VFB_ERR_CUDA, "field copy failed");
-    if (cudaStreamSynchronize(s) != cudaSuccess)
-        return setError(VFB_ERR_CUDA, "output: %s", cudaGetErrorString(cudaGetLastError()));
+    if (eBlocks)
+        enstrophyMean(partials.data() + 5ull * blocks, eBlocks, out8 + 5);
     return VFB_OK;
 }
 

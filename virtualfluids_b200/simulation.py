@@ -320,7 +320,7 @@ class Simulation:
         buffers for fast copies) when given."""
         N = len(self.levels[level]["geo"])
         if out is None:
-            out = [np.zeros(N, self.real) for _ in range(4)]
+            out = [np.empty(N, self.real) for _ in range(4)]
         elif len(out) != 4 or any(o.dtype != self.real or o.size != N or not o.flags.c_contiguous for o in out):
             raise ValueError(f"out must be four contiguous {np.dtype(self.real).name} arrays of {N} elements")
         _lib.check(_lib.lib().vfb_sim_macroscopic(self._h, level, *[o.ctypes.data for o in out], self.stream))
@@ -353,7 +353,7 @@ class Simulation:
         with fields=True, the host arrays drho, vx, vy, vz."""
         out = (ctypes.c_double * 8)()
         N = len(self.levels[level]["geo"])
-        arrays = [np.zeros(N, self.real) for _ in range(4)] if fields else [None] * 4
+        arrays = [np.empty(N, self.real) for _ in range(4)] if fields else [None] * 4
         ptrs = [None if a is None else a.ctypes.data for a in arrays]
         _lib.check(_lib.lib().vfb_sim_output(self._h, level, out, *ptrs, self.stream))
         r = {"mass": out[0], "energy": out[1], "nonfinite": int(out[2]), "kinetic_energy": out[3],
