@@ -124,9 +124,9 @@ int vfb_bgk_collision(int storage, const vfb_collision_args* args, void* stream)
 
 /*
  * Collision plan: a one-off analysis of a level's fluid-node list and
- * neighbour arrays that lets the planned kernels fetch runs of regular nodes
- * with bulk copies (cp.async.bulk) one warp tile ahead and skip the index
- * chain for them (virtualfluids_b200/csrc/collision_tiled.cu).  Building a
+ * neighbour arrays that lets the planned kernels read runs of regular nodes
+ * as contiguous memory, without the index chain
+ * (virtualfluids_b200/csrc/collision_tiled.cu).  Building a
  * plan copies the index arrays to the host once.  The planned kernels compute
  * exactly what vfb_k17_collision / vfb_bgk_collision compute; they require a
  * 16-byte aligned distributions array and the same index arrays (pointers,
@@ -490,7 +490,7 @@ typedef struct vfb_sim_params {
     double viscosity;          /* coarse-level kinematic viscosity, lattice units */
     double forces[3];          /* global acceleration */
     double quadricLimiters[3]; /* default 0.01 each (Parameter.cpp:69) */
-    int usePlan;               /* 1: the planned (bulk-copy) collision kernels */
+    int usePlan;               /* 1: the planned (tiled) collision kernels */
     int useGraphs;             /* 1: replay two coarse steps at a time from a captured CUDA graph */
     int useInitNeq;            /* 1: vfb_sim_init_level writes equilibrium plus the strain-rate part
                                   (Parameter::setUseInitNeq); the grid must carry neighborNeg */

@@ -75,18 +75,15 @@ inline Rates<float> makeRates(float omega, float qlP, float qlM, float qlD)
 // pair (3, 1/9) gives Kq = 1/3; K = 0 gives the plain transforms).
 template <class R>
 struct Sweep {
-    R vv, v2, nvv, n2vv, nv2, hm, hp, vvm, vvp;
+    R vv, v2, nvv, n2vv, hm, vvm;
     __device__ __forceinline__ Sweep(R v)
     {
         vv = v;
         v2 = v * v;
         nvv = -v;
         n2vv = R(-2) * v;
-        nv2 = -v2;
         hm = R(0.5) * (v2 - v);
-        hp = R(0.5) * (v2 + v);
         vvm = v - R(0.5);
-        vvp = v + R(0.5);
     }
 };
 
@@ -120,8 +117,7 @@ __device__ __forceinline__ void bwd(R& a, R& b, R& c, const Sweep<R>& w, typenam
     const R aK = K != 0 ? a + R(K) : a;
     const R hc = R(0.5) * c;
     const R na = fma(aK, w.hm, fma(b, w.vvm, hc));
-    // FP32 (scalar or paired): two operations fewer; hp - hm = v and
-    // vvp - vvm = 1, and the three populations sum to a
+    // (c' - a' = b + v (a + K), and the three populations sum to a)
     const R nc = na + fma(aK, w.vv, b);
     b = (a - na) - nc;
     a = na;

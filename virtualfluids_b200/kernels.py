@@ -133,7 +133,7 @@ def collision_args(dist, lat: DeviceLattice, omega: float, is_even: bool, *, for
 def collision(kernel: str, dist, lat: DeviceLattice, omega: float, is_even: bool, *, plan=None, stream=None,
               **kw) -> None:
     """One fused collide + stream pass (``kernel`` is "K17" or "BGK"); with a
-    CollisionPlan the planned (bulk-copy) kernel is used."""
+    CollisionPlan the planned (tiled) kernel is used."""
     a = collision_args(dist, lat, omega, is_even, **kw)
     L = _lib.lib()
     if plan is not None:
