@@ -32,9 +32,7 @@
 #include "adjoint_ops.gen.cuh"
 #include "capi_common.cuh"
 #include "d3q27.cuh"
-#include "pair32.cuh"
 #include "pdl.cuh"
-#include "tma.cuh"
 
 namespace vfb
 {
@@ -144,63 +142,6 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
     for (int d = 0; d < 27; ++d)
         dist[cell<R>(slot<EVEN>(d), N, L.k[loc(d)])] = f[inv(d)];
-}
-
-// The same for FP32 in paired arithmetic: thread t of a block takes the entries
-// t and t + kThreads of its 2 kThreads, whose values, tape and results it
-// handles together (k17Collide on a register pair issues about half the
-// instructions of two scalar ones, which bounded the scalar form: 31 us for the
-// channel's 522,560 nodes with or without the tape's 56 MB).
-template <bool EVEN>
-__global__ void __launch_bounds__(kThreads, 4)
-    tapeCollisionPairKernel(float* __restrict__ dist, unsigned long long N, const uint32_t* __restrict__ table,
-                            uint32_t n, const K17Rates<F2> r, float fx, float fy, float fz, float* __restrict__ tape)
-{
-    gridDependencyWait();
-    const uint32_t i = partOf<EVEN>() * (2 * kThreads) + threadIdx.x;
-    if (i >= n)
-        return;
-    const bool both = i + kThreads < n;
-    const uint32_t j = both ? i + kThreads : i;
-    F2 f[27];
-    {
-        Locs A, B;
-#pragma unroll
-        for (int l = 0; l < 8; ++l) {
-            A.k[l] = __ldg(table + (unsigned long long)l * n + i);
-            B.k[l] = __ldg(table + (unsigned long long)l * n + j);
-        }
-#pragma unroll
-        for (int d = 0; d < 27; ++d) {
-            const float* p = dist + (unsigned long long)slot<EVEN>(d) * N;
-            f[d] = F2(p[A.k[loc(d)]], p[B.k[loc(d)]]);
-        }
-    }
-    if (tape) {
-#pragma unroll
-        for (int d = 0; d < 27; ++d) {
-            float* p = tape + (unsigned long long)d * n;
-            __stcs(p + i, f[d].v.x);
-            if (both)
-                __stcs(p + j, f[d].v.y);
-        }
-    }
-    F2 drho, ux, uy, uz;
-    k17Collide<F2>(f, r, F2(fx), F2(fy), F2(fz), drho, ux, uy, uz);
-    // the locations again, rather than 16 registers held over the collision
-    Locs A, B;
-#pragma unroll
-    for (int l = 0; l < 8; ++l) {
-        A.k[l] = tma::ldgOrdered(table + (unsigned long long)l * n + i);
-        B.k[l] = tma::ldgOrdered(table + (unsigned long long)l * n + j);
-    }
-#pragma unroll
-    for (int d = 0; d < 27; ++d) {
-        float* p = dist + (unsigned long long)slot<EVEN>(d) * N;
-        p[A.k[loc(d)]] = f[inv(d)].v.x;
-        if (both)
-            p[B.k[loc(d)]] = f[inv(d)].v.y;
-    }
 }
 
 // MINB: resident blocks per SM the register allocation aims at (the reverse
@@ -727,18 +668,6 @@ int collision(R* dist, unsigned long long N, const uint32_t* nX, const uint32_t*
 {
     if (nFluid == 0)
         return VFB_OK;
-    if constexpr (sizeof(R) == 4) {
-        if (loc) {
-            const unsigned b = (nFluid + 2 * kThreads - 1) / (2 * kThreads);
-            if (even)
-                launchDependent(tapeCollisionPairKernel<true>, b, kThreads, 0, s, dist, N, loc, nFluid,
-                                pairRates(rates), fx, fy, fz, tape);
-            else
-                launchDependent(tapeCollisionPairKernel<false>, b, kThreads, 0, s, dist, N, loc, nFluid,
-                                pairRates(rates), fx, fy, fz, tape);
-            return checkLaunch("adjoint forward collision");
-        }
-    }
     const unsigned b = blocksFor(nFluid);
     if (even)
         launchDependent(tapeCollisionKernel<R, true>, b, kThreads, 0, s, dist, N, nX, nY, nZ, fluid, loc, nFluid,
