@@ -6,12 +6,13 @@
 // The two arrangements round differently, by a few units of FP32 (the shorter
 // one less).  In FP32 and FP64 storage that stays at rounding level.  A 16-bit
 // store turns it into a different code wherever a value lies next to a rounding
-// boundary, about one stored value in ten in the corner directions, so that
-// after four steps of Taylor-Green 320^3 the z velocity (little more than noise
-// there) differed by 1% and the two-level cube's FP16 populations by 1.7e-4,
-// above the bounds 16-bit results are held to from version to version.  The
-// shorter arrangement would make these storages 9% to 12% faster; they keep the
-// rounding that existing 16-bit results were made with.
+// boundary, about one stored value in ten in the corner directions: after four
+// steps of Taylor-Green 320^3 the z velocity (little more than noise there)
+// differed by 1%, the two-level cube's FP16 populations by 1.7e-4, while the
+// error against 64 bits stayed at that of the format.  The shorter arrangement
+// would make these storages 9% to 12% faster; the collision keeps the codes it
+// has stored so far (tests/test_gpu_16bit_codes.py).  The boundary lists and
+// the refinement interface have one arrangement for all storages.
 #pragma once
 
 #include "collision_math.cuh"
@@ -338,26 +339,27 @@ __device__ __forceinline__ void k17Collide(R* f, const Rates<R>& r, R fx, R fy, 
     mxxPyyPzz += (m000 - mxxPyyPzz) - R(1.5) * (vx2 * dxux + vy2 * dyuy + vz2 * dzuz);
     mxxMyy += r.minusOmega * mxxMyy - r.secondOrderCorrection * (vx2 * dxux - vy2 * dyuy);
     mxxMzz += r.minusOmega * mxxMzz - r.secondOrderCorrection * (vx2 * dxux - vz2 * dzuz);
-    m011 += r.minusOmega * m011;
-    m101 += r.minusOmega * m101;
-    m110 += r.minusOmega * m110;
+    m011 = fma(r.minusOmega, m011, m011);
+    m101 = fma(r.minusOmega, m101, m101);
+    m110 = fma(r.minusOmega, m110, m110);
 
-    // third order with quartic limiter (:404-417)
+    // third order with quartic limiter (:404-417); x - w x rounded once (as a
+    // rounded product subtracted from x it stores other codes)
     R w;
     w = fma(r.oneMinusOxyz, limiterQuotient(fabs(m111), fabs(m111) + r.qlD), r.Oxyz);
-    m111 = m111 - w * m111;
+    m111 = fma(-w, m111, m111);
     w = fma(r.oneMinusOxyyPxzz, limiterQuotient(fabs(mxxyPyzz), fabs(mxxyPyzz) + r.qlP), r.OxyyPxzz);
-    mxxyPyzz = mxxyPyzz - w * mxxyPyzz;
+    mxxyPyzz = fma(-w, mxxyPyzz, mxxyPyzz);
     w = fma(r.oneMinusOxyyMxzz, limiterQuotient(fabs(mxxyMyzz), fabs(mxxyMyzz) + r.qlM), r.OxyyMxzz);
-    mxxyMyzz = mxxyMyzz - w * mxxyMyzz;
+    mxxyMyzz = fma(-w, mxxyMyzz, mxxyMyzz);
     w = fma(r.oneMinusOxyyPxzz, limiterQuotient(fabs(mxxzPyyz), fabs(mxxzPyyz) + r.qlP), r.OxyyPxzz);
-    mxxzPyyz = mxxzPyyz - w * mxxzPyyz;
+    mxxzPyyz = fma(-w, mxxzPyyz, mxxzPyyz);
     w = fma(r.oneMinusOxyyMxzz, limiterQuotient(fabs(mxxzMyyz), fabs(mxxzMyyz) + r.qlM), r.OxyyMxzz);
-    mxxzMyyz = mxxzMyyz - w * mxxzMyyz;
+    mxxzMyyz = fma(-w, mxxzMyyz, mxxzMyyz);
     w = fma(r.oneMinusOxyyPxzz, limiterQuotient(fabs(mxyyPxzz), fabs(mxyyPxzz) + r.qlP), r.OxyyPxzz);
-    mxyyPxzz = mxyyPxzz - w * mxyyPxzz;
+    mxyyPxzz = fma(-w, mxyyPxzz, mxyyPxzz);
     w = fma(r.oneMinusOxyyMxzz, limiterQuotient(fabs(mxyyMxzz), fabs(mxyyMxzz) + r.qlM), r.OxyyMxzz);
-    mxyyMxzz = mxyyMxzz - w * mxyyMxzz;
+    mxyyMxzz = fma(-w, mxyyMxzz, mxyyMxzz);
 
     // back to single moments (:431-441)
     // (1/3)(-2 a + b + c) = (1/3)(a + b + c) - a, likewise for m002
