@@ -920,8 +920,11 @@ static int launchTiled(Op op, const vfb_collision_plan_impl& p, const vfb_collis
         case 7: return dispatchTuning<S, TileCfg<S, 128, 0, 4>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 12:
             // FP32: the K17 pass at five blocks per SM (B200, 256^3: 26.0 G node
-            // updates/s against 25.4 at four), BGK at four (25.8 against 24.0)
-            if (sizeof(S) == 4 && op == Op::K17 && t == VFB_TEMPLATE_DEFAULT)
+            // updates/s against 25.4 at four), BGK at four (25.8 against 24.0).
+            // With the BC epilogue four as well: at five it spills 64 to 84 bytes
+            // (cavities 64^3 / 128^3 / 192^3, us a step: 30.0 / 129 / 368, at
+            // five 36.2 / 146 / 426)
+            if (sizeof(S) == 4 && op == Op::K17 && t == VFB_TEMPLATE_DEFAULT && !a.epi)
                 return dispatchTiled<S, TileCfg<S, 256, 1, 5>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
             return dispatchTiled<S, TileCfg<S, 256, 1, 4>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 15:
