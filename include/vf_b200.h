@@ -582,6 +582,11 @@ int vfb_sim_adjoint_backward(vfb_simulation* sim, double seed, double* dVelocity
  * writes a cell another list reads or writes), out2[1] = 1 when the forward
  * pass taped its only segment (the backward pass recomputes nothing) */
 int vfb_sim_adjoint_schedule(const vfb_simulation* sim, int* out2);
+/* whether that schedule's backward pass takes and clears the adjoint at the
+ * cells a BC list writes in the launch that adds its contributions (1: no entry
+ * writes a cell an entry reads) or in a launch before it (0): out2[0] the
+ * velocity, no-slip and geometry lists, out2[1] the pressure lists (all of them) */
+int vfb_sim_adjoint_fused(const vfb_simulation* sim, int* out2);
 /* Parameter::setForcing (Parameter.cpp:463) on a running simulation (the next steps use
  * the new global force); no reference counterpart as an in-run setter */
 int vfb_sim_set_forces(vfb_simulation* sim, const double* forces3);

@@ -220,6 +220,7 @@ _SIGNATURES = [
     ("vfb_sim_adjoint_backward", ctypes.c_int,
      [ctypes.c_void_p, ctypes.c_double, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),
     ("vfb_sim_adjoint_schedule", ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)]),
+    ("vfb_sim_adjoint_fused", ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)]),
     ("vfb_saturated_populations", ctypes.c_int,
      [ctypes.c_int, ctypes.c_void_p, ctypes.c_ulonglong, ctypes.POINTER(ctypes.c_ulonglong), ctypes.c_void_p]),
     ("vfb_sim_saturated_populations", ctypes.c_int,

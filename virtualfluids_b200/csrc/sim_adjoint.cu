@@ -302,6 +302,12 @@ int objectiveValue(vfb_simulation& S, AdjointState& A, const R* dist, bool even,
     return VFB_OK;
 }
 
+bool isSet(const char* variable)
+{
+    const char* env = std::getenv(variable);
+    return env && env[0] == '1';
+}
+
 // Whether the post-collision lists of the adjoint (velocity, no-slip,
 // geometry) can run in one launch per step (commute): in both parities, no
 // cell a list writes (the cell of inv(d) in the other view, for each link d
@@ -310,15 +316,14 @@ int objectiveValue(vfb_simulation& S, AdjointState& A, const R* dist, bool even,
 // And whether the adjoint's gather and scatter can (fused): no cell any entry
 // writes is read by an entry, of its own list or another, and no two lists
 // write one cell.
-// VFB_ADJOINT_SEPARATE_LISTS=1 keeps one launch per list and separate gathers
-// (for comparisons).
+// For comparisons VFB_ADJOINT_SEPARATE_GATHERS=1 keeps separate gathers, and
+// VFB_ADJOINT_SEPARATE_LISTS=1 those and one launch per list.
 template <class R>
 int listsCommute(vfb_simulation& S, AdjointState& A, cudaStream_t s, bool& commute, bool& fused)
 {
     commute = fused = false;
-    if (const char* env = std::getenv("VFB_ADJOINT_SEPARATE_LISTS"))
-        if (env[0] == '1')
-            return VFB_OK;
+    if (isSet("VFB_ADJOINT_SEPARATE_LISTS"))
+        return VFB_OK;
     Level& L = *S.levels[0];
     struct Item {
         BcListDevice* list;
@@ -342,7 +347,7 @@ int listsCommute(vfb_simulation& S, AdjointState& A, cudaStream_t s, bool& commu
     if (cudaStreamSynchronize(s) != cudaSuccess)
         return cudaFail("BC list download");
     commute = locs.size() > 1; // else nothing to launch together
-    fused = true;
+    fused = !isSet("VFB_ADJOINT_SEPARATE_GATHERS");
     const unsigned long long N = L.N;
     for (int parity = 0; parity < 2; ++parity) {
         const bool even = parity == 0;
@@ -391,9 +396,8 @@ int pressureFused(vfb_simulation& S, AdjointState& A, cudaStream_t s)
 {
     Level& L = *S.levels[0];
     A.pressureFused.assign(L.pressure.size(), 0);
-    if (const char* env = std::getenv("VFB_ADJOINT_SEPARATE_LISTS"))
-        if (env[0] == '1')
-            return VFB_OK;
+    if (isSet("VFB_ADJOINT_SEPARATE_LISTS") || isSet("VFB_ADJOINT_SEPARATE_GATHERS"))
+        return VFB_OK;
     for (size_t p = 0; p < L.pressure.size(); ++p) {
         const PressureListDevice& P = *L.pressure[p];
         std::vector<int32_t> k(P.n), kN(P.n);
@@ -754,5 +758,18 @@ extern "C" int vfb_sim_adjoint_schedule(const vfb_simulation* sim, int* out2)
         return setError(VFB_ERR_CONFIGURATION, "no adjoint forward pass");
     out2[0] = sim->adjoint->listsCommute == 1 ? 1 : 0;
     out2[1] = sim->adjoint->taped ? 1 : 0;
+    return VFB_OK;
+}
+
+extern "C" int vfb_sim_adjoint_fused(const vfb_simulation* sim, int* out2)
+{
+    clearError();
+    if (!sim || !out2)
+        return setError(VFB_ERR_INVALID_ARGUMENT, "NULL argument");
+    if (!sim->adjoint || !sim->adjoint->ready)
+        return setError(VFB_ERR_CONFIGURATION, "no adjoint forward pass");
+    const AdjointState& A = *sim->adjoint;
+    out2[0] = A.listsFused ? 1 : 0;
+    out2[1] = std::all_of(A.pressureFused.begin(), A.pressureFused.end(), [](char f) { return f != 0; }) ? 1 : 0;
     return VFB_OK;
 }

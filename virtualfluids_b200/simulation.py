@@ -417,6 +417,13 @@ class Simulation:
         _lib.check(_lib.lib().vfb_sim_adjoint_schedule(self._h, out))
         return {"lists_together": bool(out[0]), "taped_forward": bool(out[1])}
 
+    def adjoint_fused(self) -> dict:
+        """Whether the backward pass of the last adjoint_forward gathers and
+        scatters in one launch: the BC lists, and every pressure list."""
+        out = (ctypes.c_int * 2)()
+        _lib.check(_lib.lib().vfb_sim_adjoint_fused(self._h, out))
+        return {"lists": bool(out[0]), "pressure": bool(out[1])}
+
     def bc_epilogue_stats(self, level: int = 0) -> tuple[int, int, int]:
         """(nodes, BC entries) the level's collision applies in its BC
         epilogue, and the entries left to the separate BC launches."""
