@@ -66,3 +66,22 @@ def test_lists_that_share_cells_are_not_fused(cuda):
     assert np.abs(dv - dv_ref).max() <= 1e-9 * np.abs(dv_ref).max()
     assert np.abs(df - df_ref).max() <= 1e-9 * np.abs(df_ref).max()
     sim.close()
+
+
+def test_fused_lists_take_no_gather_scratch(cuda, monkeypatch):
+    """27 FP64 values of every BC entry fewer on the device when nothing gathers."""
+    taken = []
+    for variable in (None, None, "VFB_ADJOINT_SEPARATE_GATHERS"):  # the first run loads the kernels too
+        if variable:
+            monkeypatch.setenv(variable, "1")
+        before = torch.cuda.mem_get_info()[0]
+        sim = make_sim(adjoint_channel_builder(128, 64, 64, (40, 26, 26, 52, 38, 38)))
+        g = sim.levels[0]
+        pb = problem(sim, 4, 2, (80, 96, 24, 40, 24, 40))
+        pb.evaluate(inlet_profile(g), G)
+        pb.gradient(1.0)
+        taken.append(before - torch.cuda.mem_get_info()[0])
+        entries = sum(len(g[k]) for k in ("velocity.k", "geometry.k", "pressure0.k"))
+        sim.close()
+    assert entries > 40000
+    assert taken[2] - taken[1] >= 0.75 * 27 * 8 * entries  # the allocator's granularity of 2 MiB a buffer

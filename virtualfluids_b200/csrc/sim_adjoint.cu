@@ -60,6 +60,10 @@ struct AdjointState {
     // their adjoints gather and scatter in one launch; the same per pressure list
     bool listsFused = false;
     std::vector<char> pressureFused;
+    bool allPressureFused() const
+    {
+        return std::all_of(pressureFused.begin(), pressureFused.end(), [](char f) { return f != 0; });
+    }
     // the forward pass recorded the tapes and BC records of its only segment:
     // the backward pass reverses them without recomputing the steps
     bool taped = false;
@@ -428,14 +432,17 @@ int ensureSegmentBuffers(vfb_simulation& S, AdjointState& A)
     DeviceBuffer* held[] = { &A.work, &A.lam, &A.tape, &A.recVelocity, &A.recNoSlip, &A.recGeometry, &A.recPressure,
                              &A.tmpVelocity, &A.tmpNoSlip, &A.tmpGeometry, &A.tmpPressure, &A.gVelocity,
                              &A.partials, &A.accForce, &A.forcePartials };
+    // a fused adjoint needs no scratch for gathered values
+    const size_t gathered = A.listsFused ? 0 : 1;
+    const size_t pressureGathered = A.allPressureFused() ? 0 : 1;
     std::vector<void*> before;
     for (DeviceBuffer* b : held)
         before.push_back(b->ptr);
     if (ensure(A.work, stateBytes) || ensure(A.lam, stateBytes) || perStep(A.tape, L.nFluid) ||
         perStep(A.recVelocity, L.velocity.n) || perStep(A.recNoSlip, L.noSlip.n) ||
         perStep(A.recGeometry, L.geometry.n) || perStep(A.recPressure, A.pressureTotal) ||
-        once(A.tmpVelocity, L.velocity.n) || once(A.tmpNoSlip, L.noSlip.n) || once(A.tmpGeometry, L.geometry.n) ||
-        once(A.tmpPressure, A.pressureTotal) ||
+        once(A.tmpVelocity, gathered * L.velocity.n) || once(A.tmpNoSlip, gathered * L.noSlip.n) ||
+        once(A.tmpGeometry, gathered * L.geometry.n) || once(A.tmpPressure, pressureGathered * A.pressureTotal) ||
         ensure(A.gVelocity, std::max<size_t>(1, 3ull * L.velocity.n * sizeof(double))) ||
         ensure(A.forcePartials, 3ull * std::max(1u, adjoint::collisionPartials(L.nFluid)) * sizeof(double)))
         return cudaFail("adjoint buffers");
@@ -770,6 +777,6 @@ extern "C" int vfb_sim_adjoint_fused(const vfb_simulation* sim, int* out2)
         return setError(VFB_ERR_CONFIGURATION, "no adjoint forward pass");
     const AdjointState& A = *sim->adjoint;
     out2[0] = A.listsFused ? 1 : 0;
-    out2[1] = std::all_of(A.pressureFused.begin(), A.pressureFused.end(), [](char f) { return f != 0; }) ? 1 : 0;
+    out2[1] = A.allPressureFused() ? 1 : 0;
     return VFB_OK;
 }
