@@ -1,7 +1,8 @@
-"""Launch forms of the planned collision and of the host copies at the sizes
-where they can go wrong: boxes below, at and above one tile, odd sizes, plans
-with and without a lane list and with nothing but one, an odd number of steps
-(the tiles run in descending order in the odd ones)."""
+"""Launch forms of the planned collision and of the output at the sizes where
+they can go wrong: boxes below, at and above one tile, odd sizes, plans with and
+without a lane list and with nothing but one, an odd number of steps (the tiles
+run in descending order in the odd ones), outputs below and above the number of
+blocks that the partial sums' buffer holds at most."""
 import numpy as np
 import pytest
 
@@ -58,29 +59,41 @@ def test_planned_equals_generic(cuda, dtype, tol, kernel, size, sphere, steps):
     assert (rel_max if dtype == "float64" else rel_l2)(got, ref) < tol
 
 
-@pytest.mark.parametrize("n", [20, 79, 80, 121])
-def test_output_copies_equal_plain_copies(cuda, n):
-    """The fields of a level below and above the size from which several
-    threads copy them (2 MiB in all), into pageable and into pinned arrays."""
+# 256 nodes a block; the output pass runs at most eight blocks an SM, the enstrophy four (B200: 1184 and 592):
+# 41 x 43 x 44 nodes (304 blocks), 103 x 43 x 44 (762, between the two), 210 x 43 x 44 (1553, above both)
+@pytest.mark.parametrize("n", [39, 101, 208])
+@pytest.mark.parametrize("inverse", [True, False])
+def test_output_equals_separate_calls(cuda, n, inverse):
+    """All values of the output against the separate passes, twice with a step
+    between, since the second call finds the first one's partial sums; a level
+    without inverse neighbours has no enstrophy section.  The sums to 1e-12 (order
+    of summation), counts and fields exactly."""
     b = MultipleGridBuilder()
-    b.addCoarseGrid(0, 0, 0, n - 1, 39, 40, 1.0)
+    b.addCoarseGrid(0, 0, 0, n, 41, 42, 1.0)
     b.buildGrids()
     b.setVelocityBoundaryCondition(SideType.PZ, 0.05, 0.0, 0.0)
+    g = dict(b.arrays()[0])
+    if not inverse:
+        del g["neighborNeg"]
     p = Parameter()
     p.set_viscosity_LB(0.01)
     p.set_storage("fp32")
-    sim = Simulation(p, b, BoundaryConditionFactory())
-    N = len(sim.levels[0]["geo"])
+    sim = Simulation(p, [g], BoundaryConditionFactory())
+    N = len(g["geo"])
     rng = np.random.default_rng(n)
-    sim.init_level(0, *[1e-3 * rng.uniform(-1, 1, N) for _ in range(4)])
-    sim.run(3)
-    pinned = [torch.zeros(N, dtype=torch.float32, pin_memory=True).numpy() for _ in range(4)]
-    sim.macroscopic(0, out=pinned)
-    for _ in range(2):
-        for a, ref in zip(sim.macroscopic(0), pinned):
-            assert np.array_equal(a, ref)
+    sim.init_level(0, *[np.where(g["geo"] == 19, 1e-3 * rng.uniform(-1, 1, N), 0.0) for _ in range(4)])
+    for steps in (3, 1):
+        sim.run(steps)
         out = sim.output(0)
-        for a, ref in zip(out["fields"], pinned):
+        for a, ref in zip(out["fields"], sim.macroscopic(0)):
             assert np.array_equal(a, ref)
-        assert out["enstrophy"] == sim.enstrophy(0)[0]
+        mass, energy, bad = sim.mass_and_energy(0)
+        kinetic, kinetic_nodes = sim.kinetic_energy(0)
+        enstrophy, enstrophy_nodes = sim.enstrophy(0) if inverse else (0.0, 0)
+        assert out["nonfinite"] == bad == 0 and out["fluid_nodes"] == len(g["fluid"])
+        assert out["kinetic_energy_nodes"] == kinetic_nodes and out["enstrophy_nodes"] == enstrophy_nodes
+        assert (enstrophy_nodes > 0) == inverse and energy > 0
+        for got, ref in ((out["mass"], mass), (out["energy"], energy), (out["kinetic_energy"], kinetic),
+                         (out["enstrophy"], enstrophy)):
+            assert abs(got - ref) <= 1e-12 * max(abs(ref), energy)
     sim.close()

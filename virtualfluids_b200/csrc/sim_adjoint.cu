@@ -91,16 +91,7 @@ void destroyAdjoint(AdjointState* a) { delete a; }
 
 namespace
 {
-cudaError_t ensure(DeviceBuffer& b, size_t bytes)
-{
-    if (b.ptr && b.bytes >= bytes)
-        return cudaSuccess;
-    if (b.ptr) {
-        cudaFree(b.ptr);
-        b.ptr = nullptr;
-    }
-    return b.allocate(bytes);
-}
+cudaError_t ensure(DeviceBuffer& b, size_t bytes) { return b.reserve(bytes); }
 
 template <class T>
 T* as(DeviceBuffer& b)

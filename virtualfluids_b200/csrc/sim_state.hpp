@@ -25,6 +25,16 @@ struct DeviceBuffer {
         bytes = n;
         return cudaMalloc(&ptr, n ? n : 1);
     }
+    // at least n bytes; the contents are lost when the buffer grows
+    cudaError_t reserve(size_t n)
+    {
+        if (ptr && bytes >= n)
+            return cudaSuccess;
+        if (ptr)
+            cudaFree(ptr);
+        ptr = nullptr;
+        return allocate(n);
+    }
     ~DeviceBuffer()
     {
         if (ptr)

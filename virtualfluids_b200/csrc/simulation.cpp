@@ -1122,7 +1122,7 @@ extern "C" int vfb_sim_output(vfb_simulation* sim, int level, double* out8, void
     // allocated its partial sums and waited for them (0.5 ms of an output call)
     const unsigned blocks = outputBlocks(L->N), eBlocks = L->nNeg.ptr ? enstrophyBlocks(L->N) : 0;
     std::vector<double> partials(5ull * blocks + 2ull * eBlocks);
-    if (!L->outPartials.ptr && L->outPartials.allocate(partials.size() * sizeof(double)) != cudaSuccess)
+    if (L->outPartials.reserve(partials.size() * sizeof(double)) != cudaSuccess)
         return setError(VFB_ERR_CUDA, "partial sums: %s", cudaGetErrorString(cudaGetLastError()));
     double* const dSums = static_cast<double*>(L->outPartials.ptr);
     int rc = outputLaunch(sim->params.storage, L->dist.ptr, L->N, geo, nX, nY, nZ,
