@@ -630,12 +630,12 @@ __global__ void __launch_bounds__(kThreads)
 // fixed-shape tree (the same order every call)
 constexpr int kReduceThreads = 256;
 __global__ void __launch_bounds__(kReduceThreads)
-    reduceKernel(const double* __restrict__ partials, unsigned blocks, int width, double* acc, double scale)
+    reduceKernel(const double* __restrict__ partials, unsigned count, int width, double* acc, double scale)
 {
     __shared__ double part[kReduceThreads];
     const int c = blockIdx.x;
     double s = 0.0;
-    for (unsigned b = threadIdx.x; b < blocks; b += kReduceThreads)
+    for (unsigned b = threadIdx.x; b < count; b += kReduceThreads)
         s += partials[(unsigned long long)width * b + c];
     part[threadIdx.x] = s;
     __syncthreads();
@@ -919,9 +919,9 @@ int objective(const R* dist, unsigned long long N, const uint32_t* nX, const uin
     return checkLaunch("objective");
 }
 
-int reducePartials(const double* partials, unsigned blocks, int width, double* acc, double scale, cudaStream_t s)
+int reducePartials(const double* partials, unsigned count, int width, double* acc, double scale, cudaStream_t s)
 {
-    reduceKernel<<<width, kReduceThreads, 0, s>>>(partials, blocks, width, acc, scale);
+    reduceKernel<<<width, kReduceThreads, 0, s>>>(partials, count, width, acc, scale);
     return checkLaunch("partial-sum reduction");
 }
 

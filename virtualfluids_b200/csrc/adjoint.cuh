@@ -122,7 +122,7 @@ int objective(const R* dist, unsigned long long N, const uint32_t* nX, const uin
               double* partials, R* lam, double seed, cudaStream_t s);
 unsigned objectiveBlocks(uint32_t n);
 
-// acc[c] += scale * sum over b of partials[width * b + c], c < width, in block order
-int reducePartials(const double* partials, unsigned blocks, int width, double* acc, double scale, cudaStream_t s);
+// acc[c] += scale * sum over b of partials[width * b + c], c < width, b < count, in that order
+int reducePartials(const double* partials, unsigned count, int width, double* acc, double scale, cudaStream_t s);
 } // namespace adjoint
 } // namespace vfb

@@ -47,7 +47,8 @@ struct AdjointState {
     DeviceBuffer tmpVelocity, tmpNoSlip, tmpGeometry, tmpPressure;
     std::vector<size_t> pressureOffset; // first entry of each pressure list in recPressure / tmpPressure
     size_t pressureTotal = 0;
-    DeviceBuffer objNodes, objW[3], partials, accForce, gVelocity;
+    DeviceBuffer objNodes, objW[3], accForce, gVelocity;
+    DeviceBuffer partials; // one per objective block
     DeviceBuffer forcePartials; // 3 per collision warp, accumulated over a backward pass
     DeviceBuffer fluidLocations; // 8 * nFluid: the fluid list's node locations (vfb_bc_locations)
     uint32_t nObj = 0;
@@ -574,7 +575,7 @@ int adjointBackward(vfb_simulation& S, AdjointState& A, double seed, double* dVe
         if (cudaGraphLaunch(it->second, s) != cudaSuccess)
             return cudaFail("segment graph launch");
     }
-    // the force adjoint: every block's sum over all steps, reduced once in block order
+    // the force adjoint: every warp's sum over all steps, reduced once in warp order
     if (const int rc = adjoint::reducePartials(as<double>(A.forcePartials), adjoint::collisionPartials(L.nFluid), 3,
                                                as<double>(A.accForce), 0.5 * L.forceFactor, s))
         return rc;
@@ -709,10 +710,10 @@ extern "C" int vfb_sim_adjoint_forward(vfb_simulation* sim, unsigned int steps, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     A.nObj = numberOfObjectiveNodes;
     const size_t n = std::max<uint32_t>(1, numberOfObjectiveNodes);
-    const unsigned partials = std::max(adjoint::collisionPartials(L.nFluid), adjoint::objectiveBlocks(A.nObj));
     if (ensure(A.objNodes, n * sizeof(uint32_t)) || ensure(A.objW[0], n * sizeof(double)) ||
         ensure(A.objW[1], n * sizeof(double)) || ensure(A.objW[2], n * sizeof(double)) ||
-        ensure(A.partials, 3ull * std::max(1u, partials) * sizeof(double)) || ensure(A.accForce, 4 * sizeof(double)))
+        ensure(A.partials, std::max(1u, adjoint::objectiveBlocks(A.nObj)) * sizeof(double)) ||
+        ensure(A.accForce, 4 * sizeof(double)))
         return cudaFail("objective buffers");
     if (numberOfObjectiveNodes) {
         const double* w[3] = { wx, wy, wz };
