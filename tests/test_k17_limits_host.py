@@ -38,3 +38,15 @@ def test_unlimited_by_infinity(precision):
     far, _ = lib_node(0, precision, f, 1.8, (1e18,) * 3, (0, 0, 0))
     inf, _ = lib_node(0, precision, f, 1.8, (np.inf,) * 3, (0, 0, 0))
     assert np.all(np.isfinite(inf)) and np.allclose(far, inf, rtol=1e-6 if precision == _lib.FP32 else 1e-14)
+
+
+@pytest.mark.parametrize("precision", [_lib.FP64, _lib.FP32])
+@pytest.mark.parametrize("limiter", [0.0, 1e-35])
+def test_limiter_zero_relaxes_fully(precision, limiter):
+    """A limiter of zero is the smallest bound (full relaxation), also at rest,
+    where the formula as written divides zero by zero."""
+    moving = np.random.default_rng(6).uniform(-0.5, 0.5, 27) * W
+    for f in (np.zeros(27), moving):
+        got, _ = lib_node(0, precision, f, 1.8, (limiter,) * 3, (0, 0, 0))
+        full, _ = lib_node(0, precision, f, 1.8, (1e-30,) * 3, (0, 0, 0))
+        assert np.all(np.isfinite(got)) and np.allclose(got, full, rtol=0, atol=1e-7 if precision == _lib.FP32 else 1e-15)
