@@ -136,8 +136,8 @@ int vfb_bgk_collision(int storage, const vfb_collision_args* args, void* stream)
 typedef struct vfb_collision_plan vfb_collision_plan;
 int vfb_collision_plan_create(int storage, const vfb_collision_args* args, vfb_collision_plan** plan, void* stream);
 int vfb_collision_plan_destroy(vfb_collision_plan* plan);
-/* out6: tiles, bulk tiles, lane-by-lane tiles, bulk-fed nodes, periodic
- * wrap nodes served inside bulk tiles, nodes collided lane by lane */
+/* out6: tiles, tiles read as contiguous runs, tiles left to the lane list, nodes
+ * of the former, periodic wrap nodes among them, nodes of the lane list */
 int vfb_collision_plan_stats(const vfb_collision_plan* plan, unsigned long long* out6);
 /* VFB_OK, or VFB_ERR_CUDA if a bounded wait of a planned kernel ran out
  * (synchronises the stream) */
@@ -156,8 +156,9 @@ int vfb_collision_plan_check(const vfb_collision_plan* plan, void* stream);
  * one byte per entry) receives 1 for the entries the epilogue applies; the
  * caller runs the remaining entries with vfb_bc_post after the collision as
  * before.  The lists' arrays must stay valid while the plan is used; nLists 0
- * removes the epilogue.  VFB_ERR_UNSUPPORTED for the direct-load and
- * per-thread pipelined tile configurations.  No reference counterpart.
+ * removes the epilogue.  VFB_ERR_UNSUPPORTED for the direct-load (but for the
+ * FP64 default, which then runs the staged kernel) and the per-thread pipelined
+ * tile configurations.  No reference counterpart.
  */
 typedef struct vfb_bc_epilogue_list {
     int kind;                   /* a post-collision VFB_BC_* kind */

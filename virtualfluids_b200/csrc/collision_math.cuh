@@ -227,10 +227,12 @@ __device__ __forceinline__ float limiterReciprocal<float>(float x)
     return approximateReciprocal(x);
 }
 // FP64: the single-precision reciprocal and two Newton-Raphson steps r (2 - x r),
-// each of which squares the relative error (2^-23, 2^-46, rounding).  A
+// each of which squares the relative error: 1.5 * 2^-23 at most (x rounded to
+// single precision, the approximation), then below 2^-44, then rounding.  A
 // collision has eight reciprocals; as divisions they made Taylor-Green 128^3
-// (two steps, B200) 345 us instead of 322, the 64^3 cavity 58.2 instead of 55.7.  x: a density or a limiter's denominator,
-// both far inside the range of FP32 (boundedLimiter).
+// (two steps, B200) 345 us instead of 322, the 64^3 cavity 58.2 instead of 55.7.
+// x: a density or a limiter's denominator, both far inside the range of FP32
+// (boundedLimiter; tests/test_gpu_k17_limits.py).
 __device__ __forceinline__ double newtonReciprocal(double x)
 {
     double r = (double)approximateReciprocal((float)x);

@@ -68,15 +68,22 @@ cudaError_t upload(T** dst, const std::vector<T>& v, cudaStream_t stream)
 
 // Tile configurations (tile width, stages, resident blocks) the library is
 // compiled for; 0 stages selects the direct-load kernel, 1 stage the paired
-// direct-load kernel.  Entry 12 (paired; four blocks per SM, five for the
-// default K17 pass) is the default for FP32, entry 19 (paired, five blocks) for
-// the 16-bit storages (B200, Taylor-Green 192^3 / 256^3: FP16 33.9 G node
-// updates per second with entry 19, 33.6 with entry 12, 33.2 with entry 20;
-// BF16 35.8 / 34.5 / 33.0; FX16 25.8 / 25.1 / 25.1 with the velocity read out)
-// and entry 11 (direct loads, 128 registers, four blocks) for FP64 (224^3: 12.1
-// G with direct loads, 11.2 with the staged entry 1; 128^3: 11.7 and 11.4: since
-// a node's collision fits 128 registers, 16 resident warps hide the loads better
-// than one tile of look-ahead does for 8).
+// direct-load kernel.  The defaults, measured on B200 by two K17 steps of one
+// Taylor-Green lattice (G node updates per second):
+//   FP32    entry 12: paired, four blocks per SM, five for the default K17 pass
+//           (launchTiled)
+//   16 bit  entry 19: paired, five blocks.  192^3 / 256^3 with entry 19, entry
+//           12 (four), entry 20 (six): FP16 32.9 / 33.7, 30.6 / 30.7, 32.4 /
+//           33.3; BF16 34.6 / 35.3, 31.9 / 31.8, 33.8 / 34.7; FX16 31.8 / 32.5,
+//           29.2 / 29.3, 31.9 / 32.8 (one entry for all three)
+//   FP64    entry 11: direct loads, 128 registers, four blocks: 16 resident warps
+//           hide the loads better than one tile of look-ahead does for the 8 of
+//           the staged entry 1.  The K17 passes without a body force fit 128
+//           registers; with one, and BGK, spill 64 to 120 bytes and still gain.
+//           us of two steps at 128^3 / 224^3, entry 11 and entry 1: K17 298 /
+//           1656 and 359 / 1970, with fields written 324 / 1763 and 402 / 2188,
+//           with a body force 326 / 1785 and 381 / 1987, with both 378 / 2025
+//           and 442 / 2394, BGK 332 / 1851 and 350 / 1934
 // VFB_TILE_CONFIG=<index> selects another one at plan creation (used to tune
 // the shape on new hardware).
 struct TileConfigInfo {

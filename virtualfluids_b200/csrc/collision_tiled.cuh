@@ -10,28 +10,28 @@
 // neighbours' neighbours).  Regular nodes are grouped into tiles covering a
 // range of T consecutive sparse indices [k0, k0+T) (T = 256, or 128 for FP64);
 // for each of the 27 directions the populations of such a range are one
-// contiguous run of memory, so the whole tile is fetched with 27 bulk copies
-// (cp.async.bulk, about 1 KB each) into shared memory while the block
-// collides the previous tile, and no index array is read for it.  A bit mask
+// contiguous run of memory, and no index array is read for it.  A bit mask
 // marks which indices of the range are members of the fluid-node list (the
 // others -- stoppers, removed or differently tagged nodes -- are skipped).
 // Nodes on a periodic wrap stay in the tiles (their wrapped locations are
 // read and written in global memory by their own lane).  Irregular nodes
 // (next to removed ones, at refinement borders) and sparse ranges go to a
-// lane list, collided one node per thread through the index chain by the
-// generic kernel.
+// lane list with a table of each node's eight locations: the direct and the
+// paired kernel collide it in their first blocks, for the others the generic
+// kernel does in a launch before them.
 //
 // Three kernels consume the plan.  In the direct kernel (the FP64 default)
 // each block takes one tile and its warps load their values from global memory
 // straight into registers; the paired kernel (the default of the FP32
 // arithmetic) does the same with two nodes a thread.  In the staged kernel
 // (FP64 with the BC epilogue, tuning configurations) each block owns
-// shared-memory stages with an mbarrier pair each; blocks of a persistent grid
-// stride over the tiles.  The arithmetic is the same k17Collide / bgkCollide
-// as the generic kernel.  Every population location
-// is read and written by exactly one node, and a thread uses only the values
-// at its own node's locations, so values a bulk copy fetches for positions no
-// thread uses may be stale without harm.
+// shared-memory stages with an mbarrier pair each, filled by 27 bulk copies a
+// tile (cp.async.bulk, about 1 KB each) while it collides the previous one;
+// blocks of a persistent grid stride over the tiles.  The arithmetic is the
+// generic kernel's.  Every population location is read and written by exactly
+// one node, and a thread uses only the values at its own node's locations, so
+// values a bulk copy fetches for positions no thread uses may be stale without
+// harm.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -919,11 +919,11 @@ static int launchTiled(Op op, const vfb_collision_plan_impl& p, const vfb_collis
         case 5: return dispatchTuning<S, TileCfg<S, 128, 4, 3>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 7: return dispatchTuning<S, TileCfg<S, 128, 0, 4>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
         case 12:
-            // FP32: the K17 pass at five blocks per SM (B200, 256^3: 26.0 G node
-            // updates/s against 25.4 at four), BGK at four (25.8 against 24.0).
-            // With the BC epilogue four as well: at five it spills 64 to 84 bytes
-            // (cavities 64^3 / 128^3 / 192^3, us a step: 30.0 / 129 / 368, at
-            // five 36.2 / 146 / 426)
+            // FP32: the K17 pass at five blocks per SM (B200, 256^3, one
+            // lattice: 27.2 G node updates/s against 26.9 at four), BGK at four
+            // (26.9 against 24.6 at five).  With the BC epilogue four as well: at
+            // five it spills 64 to 84 bytes (cavities 64^3 / 128^3 / 192^3, us a
+            // step: 30.0 / 129 / 368, at five 36.2 / 146 / 426)
             if (sizeof(S) == 4 && op == Op::K17 && t == VFB_TEMPLATE_DEFAULT && !a.epi)
                 return dispatchTiled<S, TileCfg<S, 256, 1, 5>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
             return dispatchTiled<S, TileCfg<S, 256, 1, 4>>(op, even, t, a, p.sy, p.sz, p.metaWords, stream);
